@@ -234,14 +234,12 @@ int run_vdiff2(const Dev& d, cudaStream_t s, R dt, R cnpar, const R* hn, const R
 template <class R>
 int run_tridiag(cudaStream_t s, int ncol, int kmax, int fi, int lt, const R* au, const R* bu, const R* cu,
                 const R* du, R* value) {
-  const int nt = 64;
-  const size_t smem = 2 * (size_t)(kmax + 1) * nt * sizeof(R);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(k_tridiag<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr_set = true;
+  const size_t smem = 2 * (size_t)(kmax + 1) * TRN * sizeof(R);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(k_tridiag<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
   }
-  k_tridiag<R><<<(ncol + nt - 1) / nt, nt, smem, s>>>(ncol, kmax, fi, lt, au, bu, cu, du, value);
+  k_tridiag<R><<<(ncol + TRN - 1) / TRN, TRN, smem, s>>>(ncol, kmax, fi, lt, au, bu, cu, du, value);
   return (int)cudaGetLastError();
 }
 
