@@ -38,24 +38,27 @@ WORKLOAD = ("mode-split baroclinic step (20 x integrate_2d + integrate_3d: 2D mo
 # macro step, each 3D field read or written once counted once; the 2D column heights that the sweeps
 # and the diffusion take in place of the 3D height arrays (equidistant sigma) are 1/kmax of a field
 # and not counted:
-#  * u sweeps: momentum U and V grids (u1: read f, U [+ adv in FP64, where the sum starts from a
-#    cleared array; the mixed step's vectorised first sweep starts it itself]; write fi, Di, adv.
-#    u2: read f, U, Di, adv; write adv), then the tracer pair (u1: read T, S, U; write T, S, Di.
-#    u2: read T, S, U, Di; write T, S, Di);
-#  * v sweeps: momentum v1, v2 on both grids (read f, V, Di, adv; write f, Di, adv), tracer pair v1,
-#    v2 (read T, S, V, Di; write T, S, Di);
+#  * two-sweep passes u, v: momentum U and V grids (read uu, vv; write f, Di, adv), mixed also the
+#    tracer pair (read T, S, uu, vv; write T, S, Di);
+#  * two-sweep passes v, u: momentum (read f, uu, vv, Di, adv; write adv), mixed also the tracer pair
+#    (read T, S, uu, vv, Di; write T, S);
+#  * one-sweep launches of the FP64 tracer pair: u1 (read T, S, U; write T, S, Di), u2, v1, v2 (and
+#    read Di);
 #  * w sweeps: momentum on both grids (read f, ww, hi, adv; write f, hi, adv), tracer pair (read T,
 #    S, ww, hi; write T, S, hi);
 #  * diffusion: one launch for T and S (read nuh, T, S; write T, S);
 # plus, with compensated tracer storage, the FP16 carried errors of T and S read and written by each
 # tracer launch (4 x 2 bytes = 2 words of 4 bytes).
-STAGE_LAUNCH_WORDS = {"adv_split_u": ([6, 5, 6, 5, 6, 7], [5, 5, 5, 5, 6, 7]),
-                      "adv_split_v": ([7, 7, 7, 7, 7, 7], [7, 7, 7, 7, 7, 7]),
+STAGE_LAUNCH_WORDS = {"adv_split_uv": ([5, 5], [5, 5, 7]),
+                      "adv_split_vu": ([6, 6], [6, 6, 7]),
+                      "adv_split_u": ([6, 7], [6, 7]),
+                      "adv_split_v": ([7, 7], [7, 7]),
                       "adv_split_w": ([7, 7, 7], [7, 7, 7]),
                       "tracer_vdiff": ([5], [5]),
                       "uv_momentum_3d": ([8, 8], [8, 8]),
                       "internal_pressure": ([6], [6])}
-LO_WORDS = {"adv_split_u": [0, 0, 0, 0, 2, 2], "adv_split_v": [0, 0, 0, 0, 2, 2], "adv_split_w": [0, 0, 2],
+LO_WORDS = {"adv_split_uv": [0, 0, 2], "adv_split_vu": [0, 0, 2], "adv_split_u": [2, 2], "adv_split_v": [2, 2],
+            "adv_split_w": [0, 0, 2],
             "tracer_vdiff": [2]}
 
 
@@ -68,9 +71,8 @@ def stage_words(stage: str, mixed: bool, compensated: bool) -> float:
 # DRAM bytes (read + write) per interior cell per launch of the FP32 stages, averaged over the
 # stage's launches in one macro step: ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum (one
 # kernel, up to three launches) on the 1024 x 1024 x 32 case of this workload, scaled per cell
-# (v sweeps: four momentum launches at 25.6 and two tracer-pair launches at 34.6; w sweeps: two at
-# 21.2 and the pair at 28.2; diffusion: one launch for T and S at 46.5).
-TRAFFIC_PER_CELL_F32 = {"adv_split_v": 28.6, "adv_split_w": 23.5, "tracer_vdiff": 46.5}
+# (w sweeps: two at 21.2 and the pair at 28.2; diffusion: one launch for T and S at 46.5).
+TRAFFIC_PER_CELL_F32 = {"adv_split_w": 23.5, "tracer_vdiff": 46.5}
 
 
 ERR_FIELDS = ("f3_T", "f3_S", "f3_uu", "f3_vv", "f2_z", "f2_U", "f2_V")

@@ -73,6 +73,18 @@ int step_record(getm_ctx* ctx, R dt, R* f, const R* uu, const R* vv, const R* ww
   const R half = R(0.5), one = R(1);
   // (level 0 of the heights is not read by the H-grid sweeps)
   const int nk = kmax;
+  if (two_sweeps_ok(ctx)) {
+    TwoSweep<R> t{};
+    t.flags = flags_for_tag(ctx, GETM_H_TAG);
+    t.f[0] = f;
+    t.S[0] = S;
+    t.uu = uu; t.vv = vv; t.ww = ww; t.hu = hu; t.hv = hv; t.ho = ho;
+    t.H = H;
+    for (int q = 0; q < 5; ++q) t.codes[q] = plane(q);
+    t.hs = hs; t.vs = vs; t.iters = 1;
+    t.field_out = true;
+    if ((rc = adv_two_sweeps<R>(ctx, dt, AH, gr, t, GETM_TIM_ADJ_RECORD))) return rc;
+  } else {
   GB_TIMED(GETM_TIM_ADJ_RECORD, (run_sweep_h<R, 0>(d, s, nk, dt, half, hs, AH, L(f, 1), L(f, 1), L(S, 1), L(ho, 1),
                                  L(H, 1), nullptr, L(uu, 1), L(hu, 1), gr.mask_uflux, gr.mask_uupdate,
                                  L(plane(0), 1))), "u1");
@@ -88,6 +100,7 @@ int step_record(getm_ctx* ctx, R dt, R* f, const R* uu, const R* vv, const R* ww
   GB_TIMED(GETM_TIM_ADJ_RECORD, (run_sweep_h<R, 0>(d, s, nk, dt, half, hs, AH, L(S, 1), L(S, 1), L(f, 1), L(H, 1),
                                  L(H, 1), nullptr, L(uu, 1), L(hu, 1), gr.mask_uflux, gr.mask_uupdate,
                                  L(plane(4), 1))), "u2");
+  }
   GB_TIMED(GETM_TIM_ADJ_RECORD, cudaMemcpyAsync(g, f, (size_t)n3 * sizeof(R), cudaMemcpyDeviceToDevice, s), "tape g");
   // the diffusion's result also goes to sn when the caller keeps the step outputs (only the solved
   // columns are written there -- the only ones the adjoint diffusion reads)

@@ -1604,6 +1604,20 @@ int integrate_3d(getm_ctx* ctx, getm_bc_state* st, int n) {
       const bool cols = (split == GETM_HALFSPLIT || split == GETM_FULLSPLIT) && is_split_scheme(hor) &&
                         is_split_scheme(ver);
       const unsigned h2d = cols ? 7u : 0u;
+      // HALFSPLIT without vertical sub-iterations: the two-sweep passes take uu, vv, ww themselves
+      // and form the advected velocities and the transports of the control volumes (no set-up pass)
+      const bool direct = cols && split == GETM_HALFSPLIT && ip[I_ADV_VER_ITERS] <= 1 &&
+                          two_sweeps_ok(ctx);
+      if (direct) {
+        for (int m = 1; m <= 2; ++m) {
+          const R3* h = CH(m == 1 ? COL_HUN : COL_HVN);
+          if ((rc = do_adv3d<R3>(ctx, R3(st->par[P_DT]), nullptr, f3[UU], f3[VV], f3[WW],
+                                 CH(m == 1 ? COL_HUA_U : COL_HUA_V), CH(m == 1 ? COL_HVA_U : COL_HVA_V), h, h, split, hor,
+                                 ver, R3(0), m == 1 ? GETM_U_TAG : GETM_V_TAG, nullptr, f3[m == 1 ? UUEX : VVEX], 1,
+                                 false, nullptr, h2d, m)))
+            return rc;
+        }
+      } else {
       const unsigned skip = cols ? ((1u << 4) | (1u << 5) | (1u << 11) | (1u << 12)) : 0u;
       R3* wv = sizeof(R3) == 4 ? w + 7 * n3 : w;
       R3 *fadv = w, *ua = w + n3, *va = w + 2 * n3, *wa = w + 3 * n3, *hua = w + 4 * n3, *hva = w + 5 * n3;
@@ -1626,6 +1640,7 @@ int integrate_3d(getm_ctx* ctx, getm_bc_state* st, int n) {
       if ((rc = do_adv3d<R3>(ctx, R3(st->par[P_DT]), fadvv, uav, vav, wav, huav, hvav, hov, hov, split, hor, ver,
                              R3(0), GETM_V_TAG, nullptr, f3[VVEX], ip[I_ADV_VER_ITERS], false, nullptr, h2d)))
         return rc;
+      }
     }
     if ((rc = bc3<R3>(ctx, st, BC3_STRESSES, GETM_TIM_BC3D))) return rc;
     // m3d.F90:570-575: gotm() with PARABOLIC_VISCOSITY (CONSTANT_VISCOSITY leaves num, nuh)
@@ -1669,7 +1684,7 @@ int integrate_3d(getm_ctx* ctx, getm_bc_state* st, int n) {
                "top-level salinity");
       if ((rc = do_adv3d_pair<R3>(ctx, dt, f3[TT], f3[SS], f3[UU], f3[VV], f3[WW], CH(COL_HUN), CH(COL_HVN),
                                   CH(COL_HO), ip[I_TEMP_HOR], ip[I_TEMP_VER], R3(st->par[P_TEMP_AH]), tlo, slo,
-                                  7u)))
+                                  7u, (__half*)((R3*)ctx->bc_scr3 + 4 * n3))))  // (a slot free at this point)
         return rc;
       if (radn && (rc = temp_sources(s_top))) return rc;
       // the two diffusion solves in one launch (shared hn, nuh); the elimination coefficients of

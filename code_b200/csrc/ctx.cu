@@ -44,6 +44,13 @@ __global__ void k_build_masks(Dev d, const int32_t* __restrict__ az, const int32
   // U grid u-flux = mask_updateH(i+1,j); V grid v-flux = mask_updateH(i,j+1)
   planes[P_UFLUX_U * n + c] = !last_i && az[c + 1] == 1;
   planes[P_VFLUX_V * n + c] = !last_j && az[c + d.sj] == 1;
+  auto pack = [&](int fu, int pu, int fv, int pv) {
+    return (uint8_t)((planes[fu * n + c] ? ADV_FU : 0) | (planes[pu * n + c] ? ADV_PU : 0) |
+                     (planes[fv * n + c] ? ADV_FV : 0) | (planes[pv * n + c] ? ADV_PV : 0));
+  };
+  planes[P_FLAGS_H * n + c] = pack(P_UFLUX, P_UPDATEH, P_VFLUX, P_UPDATEH);
+  planes[P_FLAGS_U * n + c] = pack(P_UFLUX_U, P_UUPDATEU, P_XFLUX, P_UFLUX);
+  planes[P_FLAGS_V * n + c] = pack(P_XFLUX, P_VFLUX, P_VFLUX_V, P_VUPDATEV);
 }
 
 int run_build_masks(const Dev& d, cudaStream_t s, const int32_t* az, const int32_t* au, const int32_t* av,
@@ -59,17 +66,74 @@ int run_build_masks(const Dev& d, cudaStream_t s, const int32_t* az, const int32
 using namespace gb;
 
 // ---------------------------------------------------------------------------------------------
+// u/2 v/2 | w | v/2 u/2 (advection_3d.F90:439-537) as two horizontal passes (adv_fused.cuh) around
+// the vertical sweep. The caller has checked the schemes. slot: the timer of every launch, or -1 for
+// each stage's own.
+template <class R>
+int adv_two_sweeps(getm_ctx* ctx, R dt, R AH, const getm_adv_grid& g, const TwoSweep<R>& t, int slot) {
+  const Dev& d = ctx->dev;
+  cudaStream_t s = ctx->stream;
+  const long long sk = d.sk;
+  auto L = [&](auto* p) { return p ? p + sk : p; };
+  const int nf = t.f[1] ? 2 : 1;
+  AdvPass<R> a;
+  a.U = L(t.uu);
+  a.V = L(t.vv);
+  a.du2d = t.h2d & 1u;
+  a.dv2d = t.h2d & 2u;
+  a.DU = a.du2d ? t.hu : L(t.hu);
+  a.DV = a.dv2d ? t.hv : L(t.hv);
+  a.flags = t.flags;
+  a.adv = L(t.adv);
+  a.mom = t.mom;
+  AdvPass<R> b = a;
+  a.di2d = t.h2d & 4u;
+  a.Di_src = a.di2d ? t.ho : L(t.ho);
+  a.Di_dst = L(t.H);
+  b.Di_src = L(t.H);
+  b.Di_dst = L(t.hires);
+  for (int n = 0; n < nf; ++n) {
+    a.src[n] = L((const R*)t.f[n]);
+    a.dst[n] = L(t.S[n]);
+    a.lo_src[n] = L((const __half*)t.lo[n]);
+    a.lo_dst[n] = L(t.lo_s[n]);
+    b.src[n] = L((const R*)t.S[n]);
+    b.dst[n] = t.field_out ? L(t.f[n]) : nullptr;
+    b.lo_src[n] = L((const __half*)t.lo_s[n]);
+    b.lo_dst[n] = L(t.lo[n]);
+  }
+  a.code_u = L(t.codes[0]);
+  a.code_v = L(t.codes[1]);
+  b.code_v = L(t.codes[3]);
+  b.code_u = L(t.codes[4]);
+  auto tim = [&](int own) { return slot >= 0 ? slot : own; };
+  GB_TIMED(tim(GETM_TIM_TRACER_UV), run_adv_pass<R>(d, s, false, d.kmax, dt, t.hs, AH, a), "u, v");
+  if (t.kshift == 1)  // the W-grid vertical sweep also reads level 0 of the field
+    GB_TRY(cudaMemcpyAsync(t.S[0], t.f[0], (size_t)sk * sizeof(R), cudaMemcpyDeviceToDevice, s), "copy f(0)");
+  if (d.kmax > 1 && t.vs != NOADV) {
+    if (nf == 2)
+      GB_TIMED(tim(GETM_TIM_ADV_W), run_sweep_w2<R>(d, s, dt, R(1), t.vs, t.S[0], t.S[1], t.H, t.ww, g.az, t.lo_s[0], t.lo_s[1]), "w");
+    else
+      GB_TIMED(tim(GETM_TIM_ADV_W), run_sweep_w<R>(d, s, dt, R(1), t.vs, t.kshift, t.iters, t.S[0], t.S[0], t.S[0], t.H, t.adv,
+                                                   t.ww, g.az, ctx->cnt, t.codes[2], t.lo_s[0], t.mom), "w");
+  }
+  GB_TIMED(tim(GETM_TIM_TRACER_WVU), run_adv_pass<R>(d, s, true, d.kmax, dt, t.hs, AH, b), "v, u");
+  return GETM_OK;
+}
+template int adv_two_sweeps<double>(getm_ctx*, double, double, const getm_adv_grid&, const TwoSweep<double>&, int);
+template int adv_two_sweeps<float>(getm_ctx*, float, float, const getm_adv_grid&, const TwoSweep<float>&, int);
+
 // do_advection_3d (advection_3d.F90:279-566) on device pointers (level-0 origin).
 template <class R>
 int do_adv3d(getm_ctx* ctx, R dt, R* f, const R* uu, const R* vv, const R* ww, const R* hu,
                     const R* hv, const R* ho, const R* hn, int split, int hs, int vs, R AH, int tag, R* hires,
-                    R* advres, int iters, bool field_out, __half* lo, unsigned h2d) {
+                    R* advres, int iters, bool field_out, __half* lo, unsigned h2d, int mom) {
   (void)hn;
   if (!ctx) return GETM_ERR_ARG;
   if (!ctx->adv_ready) return fail(ctx, GETM_ERR_STATE, "getm_init_advection has not been called");
   getm_adv_grid g;
   if (!grid_for_tag(ctx, tag, &g)) return fail(ctx, GETM_ERR_ARG, "do_advection_3d: tag is invalid");
-  if (!f || !ho) return fail(ctx, GETM_ERR_ARG, "do_advection_3d: null field");
+  if ((!f && !mom) || !ho) return fail(ctx, GETM_ERR_ARG, "do_advection_3d: null field");
   if (hs != NOADV && !is_split_scheme(hs)) {
     if (hs == UPSTREAM_2DH || hs == 7 || hs == 8 || hs == 9)
       return fail(ctx, GETM_ERR_UNSUPPORTED, "do_advection_3d: 2DH schemes are not provided");
@@ -89,7 +153,16 @@ int do_adv3d(getm_ctx* ctx, R dt, R* f, const R* uu, const R* vv, const R* ww, c
   int rc = ensure_scratch(ctx, bytes3);
   if (rc) return rc;
   R* S = (R*)ctx->scr[0];
-  R* H = hires ? hires : (R*)ctx->scr[1];
+  // HALFSPLIT as two-sweep passes, unless the final heights are to overwrite an array the passes
+  // read (they keep their own height array until the end)
+  auto apart = [&](const R* p, bool plane) {
+    return !hires || !p || hires + n3 <= p || p + (plane ? n2d(d) : n3) <= hires;
+  };
+  const bool passes = split == GETM_HALFSPLIT && hs != NOADV && vs != NOADV && two_sweeps_ok(ctx) && apart(f, false) && apart(uu, false) && apart(vv, false) &&
+                      apart(ww, false) && apart(hu, h2d & 1u) && apart(hv, h2d & 2u) && apart(ho, h2d & 4u);
+  if (mom && (!passes || !advres || iters > 1))
+    return fail(ctx, GETM_ERR_STATE, "do_advection_3d: momentum advection needs the two-sweep passes");
+  R* H = hires && !passes ? hires : (R*)ctx->scr[1];
   const bool needs_adv = (hs != NOADV && vs != NOADV && (split == GETM_NOSPLIT || split == GETM_HVSPLIT)) ||
                          (hs != NOADV && vs == NOADV && split == GETM_NOSPLIT);
   R* A = advres ? advres : (needs_adv ? (R*)ctx->scr[2] : nullptr);
@@ -101,6 +174,7 @@ int do_adv3d(getm_ctx* ctx, R dt, R* f, const R* uu, const R* vv, const R* ww, c
   // (the layer heights of equidistant sigma coordinates); only the FULLSPLIT and HALFSPLIT sweeps
   // take them
   if (h2d && (!split_first_u || hires)) return fail(ctx, GETM_ERR_STATE, "do_advection_3d: 2D heights need a split");
+  // (the two-sweep passes start the sum like the vectorised u sweep: level 0 is cleared here)
   if (A) GB_TRY(cudaMemsetAsync(A, 0, split_first_u ? (size_t)sk * sizeof(R) : bytes3, s), "memset adv");
   auto L = [&](auto* p, int k) { return p + (long long)k * sk; };
   const R half = R(0.5), one = R(1);
@@ -146,6 +220,23 @@ int do_adv3d(getm_ctx* ctx, R dt, R* f, const R* uu, const R* vv, const R* ww, c
       return fail(ctx, GETM_ERR_ARG, "do_advection: split is invalid");
     }
     return GETM_OK;
+  }
+  if (passes) {
+    TwoSweep<R> t{};
+    t.flags = flags_for_tag(ctx, tag);
+    t.f[0] = f;
+    t.S[0] = S;
+    t.lo[0] = (lo && field_out && sizeof(R) == 4) ? lo : nullptr;
+    t.lo_s[0] = t.lo[0] ? (__half*)ctx->scr[2] : nullptr;
+    t.uu = uu; t.vv = vv; t.ww = ww; t.hu = hu; t.hv = hv; t.ho = ho;
+    t.H = H;
+    t.hires = hires;
+    t.adv = A;
+    t.hs = hs; t.vs = vs; t.iters = iters; t.kshift = kshift; t.mom = mom;
+    t.field_out = field_out;
+    t.h2d = h2d;
+    if (hires) GB_TRY(cudaMemcpyAsync(hires, ho, (size_t)sk * sizeof(R), cudaMemcpyDeviceToDevice, s), "copy ho(0)");
+    return adv_two_sweeps<R>(ctx, dt, AH, g, t, -1);
   }
   R* Al = A ? L(A, 1) : nullptr;
   // compensated storage of the tracer (FP32; the FULLSPLIT and HALFSPLIT sequences, whose updates
@@ -211,7 +302,8 @@ int do_adv3d(getm_ctx* ctx, R dt, R* f, const R* uu, const R* vv, const R* ww, c
 // same sweeps as do_adv3d's HALFSPLIT branch for each field, with the heights hi evolved once.
 template <class R>
 int do_adv3d_pair(getm_ctx* ctx, R dt, R* fa, R* fb, const R* uu, const R* vv, const R* ww, const R* hu,
-                  const R* hv, const R* ho, int hs, int vs, R AH, __half* lo_a, __half* lo_b, unsigned h2d) {
+                  const R* hv, const R* ho, int hs, int vs, R AH, __half* lo_a, __half* lo_b, unsigned h2d,
+                  __half* lo_scr) {
   getm_adv_grid g;
   grid_for_tag(ctx, GETM_H_TAG, &g);
   const Dev& d = ctx->dev;
@@ -226,6 +318,31 @@ int do_adv3d_pair(getm_ctx* ctx, R dt, R* fa, R* fb, const R* uu, const R* vv, c
   auto L = [&](auto* p, int k) { return p ? p + (long long)k * sk : p; };
   const R half = R(0.5), one = R(1);
   const int nk = kmax;
+  if (sizeof(R) == 8) lo_a = lo_b = nullptr;
+  // FP64: two fields' windows at 96 registers per thread lose to the one-sweep kernels where the domain
+  // fills the GPU (512x512x30: 1.02 against 0.86 ms for the four sweeps); below, four launches fewer and
+  // more warps win (step of 128x128x20: 1.43 against 1.45 ms; 200x180x25: equal)
+  const bool small = n3d(d) <= (1LL << 19);
+  if ((sizeof(R) == 4 || small) && two_sweeps_ok(ctx) && !lo_a == !lo_b && (!lo_a || lo_scr)) {
+    TwoSweep<R> t{};
+    t.flags = flags_for_tag(ctx, GETM_H_TAG);
+    t.f[0] = fa;
+    t.f[1] = fb;
+    t.S[0] = Sa;
+    t.S[1] = Sb;
+    t.lo[0] = lo_a;
+    t.lo[1] = lo_b;
+    if (lo_a) {
+      t.lo_s[0] = lo_scr;
+      t.lo_s[1] = lo_scr + n3d(d);
+    }
+    t.uu = uu; t.vv = vv; t.ww = ww; t.hu = hu; t.hv = hv; t.ho = ho;
+    t.H = H;
+    t.hs = hs; t.vs = vs; t.iters = 1;
+    t.field_out = true;
+    t.h2d = h2d;
+    return adv_two_sweeps<R>(ctx, dt, AH, g, t, -1);
+  }
   __half* la = L(lo_a, 1);
   __half* lb = L(lo_b, 1);
   // h2d as in do_adv3d: hu, hv, ho as 2D arrays of column values
@@ -250,16 +367,18 @@ int do_adv3d_pair(getm_ctx* ctx, R dt, R* fa, R* fb, const R* uu, const R* vv, c
   return GETM_OK;
 }
 template int do_adv3d_pair<double>(getm_ctx*, double, double*, double*, const double*, const double*, const double*,
-                                   const double*, const double*, const double*, int, int, double, __half*, __half*, unsigned);
+                                   const double*, const double*, const double*, int, int, double, __half*, __half*, unsigned,
+                                   __half*);
 template int do_adv3d_pair<float>(getm_ctx*, float, float*, float*, const float*, const float*, const float*,
-                                  const float*, const float*, const float*, int, int, float, __half*, __half*, unsigned);
+                                  const float*, const float*, const float*, int, int, float, __half*, __half*, unsigned,
+                                  __half*);
 
 template int do_adv3d<double>(getm_ctx*, double, double*, const double*, const double*, const double*,
                                const double*, const double*, const double*, const double*, int, int, int, double,
-                               int, double*, double*, int, bool, __half*, unsigned);
+                               int, double*, double*, int, bool, __half*, unsigned, int);
 template int do_adv3d<float>(getm_ctx*, float, float*, const float*, const float*, const float*, const float*,
                              const float*, const float*, const float*, int, int, int, float, int, float*, float*,
-                             int, bool, __half*, unsigned);
+                             int, bool, __half*, unsigned, int);
 
 template <class R>
 static int sweep_h_api(getm_ctx* ctx, int dir, int nk, R dt, const R* f, R* fi, R* Di, R* adv, const R* U,
@@ -459,8 +578,8 @@ int getm_ctx_take_warnings(getm_ctx* ctx, int64_t* n_warnings) {
 const char* getm_ctx_last_error(const getm_ctx* ctx) { return ctx ? ctx->err.c_str() : "null context"; }
 
 static const char* kTimerNames[GETM_NTIMERS] = {"adv_split_u", "adv_split_v", "adv_split_w", "adv_finalise",
-                                                 "tracer_vdiff", "copy", "tracer_fused_uv",
-                                                 "tracer_fused_wvu", "mode_split_2d", "macro_3d_other", "internal_pressure",
+                                                 "tracer_vdiff", "copy", "adv_split_uv",
+                                                 "adv_split_vu", "mode_split_2d", "macro_3d_other", "internal_pressure",
                                                  "uv_momentum_3d", "tracer_record", "tracer_adjoint", "reserved14",
                                                  "reserved15"};
 

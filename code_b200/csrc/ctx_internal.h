@@ -12,7 +12,9 @@
 #define GB_NCOUNTERS 8
 
 namespace gb {
-enum MaskPlane { P_UPDATEH = 0, P_UFLUX, P_VFLUX, P_XFLUX, P_UUPDATEU, P_VUPDATEV, P_UFLUX_U, P_VFLUX_V, NPLANES };
+enum MaskPlane { P_UPDATEH = 0, P_UFLUX, P_VFLUX, P_XFLUX, P_UUPDATEU, P_VUPDATEV, P_UFLUX_U, P_VFLUX_V,
+                 // the masks of the T, U and V grids packed into one byte per cell (ADV_* bits)
+                 P_FLAGS_H, P_FLAGS_U, P_FLAGS_V, NPLANES };
 
 static inline long long n2d(const Dev& d) { return d.sj * (long long)d.nj(); }
 static inline long long n3d(const Dev& d) { return d.sk * (long long)(d.kmax + 1); }
@@ -167,20 +169,50 @@ static inline bool grid_for_tag(const getm_ctx* ctx, int tag, getm_adv_grid* g) 
   }
 }
 
+static inline const uint8_t* flags_for_tag(const getm_ctx* ctx, int tag) {
+  const int p = tag == GETM_U_TAG ? P_FLAGS_U : tag == GETM_V_TAG ? P_FLAGS_V : P_FLAGS_H;
+  return ctx->planes + p * n2d(ctx->dev);
+}
+// The two-sweep passes (adv_fused.cuh) serve a domain: 32-bit in-plane offsets, a grid z of levels.
+static inline bool two_sweeps_ok(const getm_ctx* ctx) {
+  return vector_sweeps_enabled() && ctx->dev.kmax >= 1 && ctx->dev.kmax <= 65535 && n2d(ctx->dev) < (1LL << 31);
+}
 
 // do_advection_3d (advection_3d.F90:120-598) on device pointers; defined in ctx.cu. lo: the
 // tracer's compensated storage (FP32, FULLSPLIT / HALFSPLIT; null = none). h2d: bit 0 hu, bit 1 hv,
 // bit 2 ho are 2D arrays of values shared by every level of a column (FULLSPLIT / HALFSPLIT only).
+// mom 1 / 2 (adv_two_sweeps only, with advres): the momentum advection of the U / V grid from the
+// 3D transports uu, vv and the T points' ww -- f is not read (null) and only advres comes out.
 template <class R>
 int do_adv3d(getm_ctx* ctx, R dt, R* f, const R* uu, const R* vv, const R* ww, const R* hu, const R* hv,
              const R* ho, const R* hn, int split, int hs, int vs, R AH, int tag, R* hires, R* advres, int iters,
-             bool field_out = true, __half* lo = nullptr, unsigned h2d = 0);
+             bool field_out = true, __half* lo = nullptr, unsigned h2d = 0, int mom = 0);
 // Two tracers advected together with HALFSPLIT on the H grid (ctx.cu); the caller has checked that
-// hs is a split scheme, vs a split scheme or NOADV, and adv_ver_iterations = 1.
+// hs is a split scheme, vs a split scheme or NOADV, and adv_ver_iterations = 1. lo_scr: room for the
+// carried errors of both between the passes (2 n3 of them; null without lo_a, lo_b).
 template <class R>
 int do_adv3d_pair(getm_ctx* ctx, R dt, R* fa, R* fb, const R* uu, const R* vv, const R* ww, const R* hu,
                   const R* hv, const R* ho, int hs, int vs, R AH, __half* lo_a = nullptr, __half* lo_b = nullptr,
-                  unsigned h2d = 0);
+                  unsigned h2d = 0, __half* lo_scr = nullptr);
+
+// Level-0 origins of the arrays of one HALFSPLIT advection as two-sweep passes (adv_two_sweeps).
+template <class R>
+struct TwoSweep {
+  R* f[2];                 // fields, in and out (second: null for one)
+  R* S[2];                 // the fields between the passes
+  __half *lo[2], *lo_s[2]; // carried errors (null: none), and between the passes
+  const uint8_t* flags;    // the grid's packed masks
+  const R *uu, *vv, *ww, *hu, *hv, *ho;
+  R *H, *hires, *adv;      // heights between the passes; final heights and flux sum (may be null)
+  uint8_t* codes[5];       // limiter branches of the five sweeps (null: not recorded)
+  int hs, vs, iters, kshift, mom;
+  bool field_out;
+  unsigned h2d;
+};
+
+// HALFSPLIT as two horizontal passes around the vertical sweep (ctx.cu)
+template <class R>
+int adv_two_sweeps(getm_ctx* ctx, R dt, R AH, const getm_adv_grid& g, const TwoSweep<R>& t, int slot);
 
 // Tracer step: do_advection_3d(H_TAG) then the implicit vertical diffusion (ctx.cu).
 template <class R>

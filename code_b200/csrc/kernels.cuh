@@ -17,7 +17,7 @@ namespace gb {
 // evaluates the same interface values with fewer instructions: the ratio-based limiters are
 // rewritten without the ratio (L(r)*deltaf from the magnitudes |deltafu|, |deltaf|, which equals
 // the reference's value in exact arithmetic) and the remaining divisions by face quantities use
-// the fast reciprocal (__fdividef, <= 2 ulp).
+// the fast reciprocal (__fdividef or fdiv_fast, <= 2 ulp).
 
 template <class R>
 __device__ __forceinline__ R qdiv(R a, R b) {
@@ -39,7 +39,7 @@ __device__ __forceinline__ Pdm32 pdm32(float cfl, float a, float b) {
   const float omc = __fsub_rn(1.f, cfl);
   const float x = __fmul_rn(1.f / 6.f, __fsub_rn(1.f, __fmul_rn(2.f, cfl)));
   Pdm32 p;
-  p.v1 = __fdividef(__fmul_rn(a, omc), __fadd_rn(cfl, 1.e-10f));
+  p.v1 = fdiv_fast(__fmul_rn(a, omc), __fadd_rn(cfl, 1.e-10f));
   p.v2 = __fmul_rn(__fmul_rn(0.5f, omc), __fmaf_rn(__fadd_rn(0.5f, x), b, __fmul_rn(__fsub_rn(0.5f, x), a)));
   return p;
 }
@@ -168,7 +168,7 @@ __device__ __forceinline__ R fv_update(R hio, R dh, R hin, R fio, R dt, R advn) 
     return (hio * fio - dt * advn) / hin;
   } else {
     (void)hio;
-    return __fadd_rn(fio, __fdividef(__fmaf_rn(fio, dh, -__fmul_rn(dt, advn)), hin));
+    return __fadd_rn(fio, fdiv_fast(__fmaf_rn(fio, dh, -__fmul_rn(dt, advn)), hin));
   }
 }
 
@@ -206,7 +206,7 @@ __device__ __forceinline__ R fv_update_lo(R hio, R dh, R hin, R fio, R dt, R adv
     return fv_update<R>(hio, dh, hin, fio, dt, advn);
   } else {
     (void)hio;
-    return add_comp_scaled(fio, __fdividef(__fmaf_rn(fio, dh, -__fmul_rn(dt, advn)), hin), slo);
+    return add_comp_scaled(fio, fdiv_fast(__fmaf_rn(fio, dh, -__fmul_rn(dt, advn)), hin), slo);
   }
 }
 // the same on the FP16 array of the carried errors at element p
@@ -247,7 +247,7 @@ __device__ __forceinline__ float face_flux_f32(float Uf, float DUf, float fm1, f
     const float fuu = pos ? fm1 : f2;
     const float fd = pos ? f1 : f0;
     const bool lim = pos ? mm1 : mp1;
-    const float cfl = __fdividef(fabsf(Uf) * cdx, DUf);
+    const float cfl = fdiv_fast(fabsf(Uf) * cdx, DUf);
     float val;
     if constexpr (S == P2_PDM) {
       const float df = fd - fu, du = fu - fuu;
@@ -662,7 +662,7 @@ __global__ void __launch_bounds__(TVX * TVY, sizeof(R) == 4 ? (NF == 1 ? 8 : 6) 
 template <class R>
 __device__ __forceinline__ R wface_cfl(R w, R dti, R hk, R hkp1) {
   if constexpr (sizeof(R) == 8) return fabs(w) * dti / (R(0.5) * (hk + hkp1));
-  else return __fdividef(2.f * fabsf(w) * dti, hk + hkp1);
+  else return fdiv_fast(2.f * fabsf(w) * dti, hk + hkp1);
 }
 
 template <class R, int S, bool REC = false>
@@ -681,7 +681,9 @@ __device__ __forceinline__ R wface_s(int k, int kshift, int kmax, R dti, R w, R 
   return w * fu;
 }
 
-template <class R, int S, bool REC>
+// MOM 1 / 2: the vertical velocity of the U / V grid's columns, the mean of ww at the two T points
+// (0 at level 0), formed here.
+template <class R, int S, bool REC, int MOM = 0>
 __global__ void __launch_bounds__(128) k_sweep_w(Dev d, R dt, R splitfac, int kshift,
                                                  const R* f, const R* fi_src, R* fi_dst, R* hi, R* adv,
                                                  const R* __restrict__ ww,
@@ -698,7 +700,10 @@ __global__ void __launch_bounds__(128) k_sweep_w(Dev d, R dt, R splitfac, int ks
   const bool fi_is_f = (fi_src == f);
   auto F = [&](int k) -> R { return (k >= 0 && k <= kmax) ? f[c + k * sk] : R(0); };
   auto H = [&](int k) -> R { return (k >= 0 && k <= kmax) ? hi[c + k * sk] : R(0); };
-  auto W = [&](int k) -> R { return (k <= kmax) ? ww[c + k * sk] : R(0); };
+  auto W = [&](int k) -> R {
+    if constexpr (MOM == 0) return (k <= kmax) ? ww[c + k * sk] : R(0);
+    else return (k >= 1 && k <= kmax) ? R(0.5) * (ww[c + k * sk] + ww[c + (MOM == 1 ? 1 : d.sj) + k * sk]) : R(0);
+  };
   R wprev = R(0);  // wflux(k-1); wflux(0) = 0 unless W_TAG computes face 0
   if (kshift == 1) {
     uint8_t cd = 0;

@@ -7,6 +7,7 @@
 
 #include "kernels.cuh"
 #include "sweeps_vec.cuh"
+#include "adv_fused.cuh"
 
 namespace gb {
 
@@ -149,6 +150,89 @@ int run_sweep_h(const Dev& d, cudaStream_t s, int nk, R dt, R splitfac, int sche
   });
 }
 
+// Cells per lane of the two-sweep passes. FP32: four where every row and level starts on a 16-byte
+// boundary (two for a tracer pair: registers), two on an 8-byte boundary, else one. FP64: one (two-cell
+// lanes need 150 registers and measured 12% slower; a warp's row access is 256 bytes either way).
+template <class R>
+int run_adv_pass(const Dev& d, cudaStream_t s, bool vu, int nk, R dt, int scheme, R AH, const AdvPass<R>& a) {
+  if (nk <= 0) return 0;
+  const bool two = vu ? a.src[1] != nullptr : a.dst[1] != nullptr, rec = a.code_u != nullptr;
+  const bool lo = sizeof(R) == 4 && a.lo_src[0] != nullptr;
+  if ((two && (a.adv || rec || a.mom)) || (rec && (a.adv || a.mom || lo)) || nk > 65535 ||
+      d.sj * (long long)d.nj() >= (1LL << 31))
+    return (int)cudaErrorInvalidValue;
+  AdvC<R> C;
+  C.u = sweep_consts<R>(d, 0, dt, R(0.5), AH);
+  C.v = sweep_consts<R>(d, 1, dt, R(0.5), AH);
+  C.u.skdu = a.du2d ? 0 : d.sk;
+  C.v.skdu = a.dv2d ? 0 : d.sk;
+  C.u.skdi = a.di2d ? 0 : d.sk;
+  C.U = a.U; C.DU = a.DU; C.V = a.V; C.DV = a.DV; C.Di_src = a.Di_src; C.Di_dst = a.Di_dst; C.adv = a.adv;
+  C.flags = a.flags; C.code_u = a.code_u; C.code_v = a.code_v;
+  auto aligned = [&](int n) {
+    if (d.sj % n != 0 || (nk > 1 && d.sk % n != 0)) return false;
+    for (const void* p : {(const void*)a.src[0], (const void*)a.src[1], (const void*)a.dst[0], (const void*)a.dst[1],
+                          (const void*)a.U, (const void*)a.DU, (const void*)a.V, (const void*)a.DV,
+                          (const void*)a.Di_src, (const void*)a.Di_dst, (const void*)a.adv})
+      if (reinterpret_cast<uintptr_t>(p) % (n * sizeof(R)) != 0) return false;
+    for (const void* p : {(const void*)a.flags, (const void*)a.code_u, (const void*)a.code_v})
+      if (reinterpret_cast<uintptr_t>(p) % n != 0) return false;
+    for (const void* p : {(const void*)a.lo_src[0], (const void*)a.lo_src[1], (const void*)a.lo_dst[0],
+                          (const void*)a.lo_dst[1]})
+      if (reinterpret_cast<uintptr_t>(p) % (2 * n) != 0) return false;
+    return true;
+  };
+  return dispatch_scheme(scheme, [&](auto sc) {
+    constexpr int S = decltype(sc)::value;
+    auto launch = [&](auto nf, auto nn, auto recc, auto loc, auto momc) -> int {
+      constexpr int NF = decltype(nf)::value, N = decltype(nn)::value, MOM = decltype(momc)::value;
+      constexpr bool REC = decltype(recc)::value, LO = decltype(loc)::value;
+      AdvF<R, NF> F;
+      for (int n = 0; n < NF; ++n) {
+        F.src[n] = a.src[n];
+        F.dst[n] = a.dst[n];
+        F.lo_src[n] = a.lo_src[n];
+        F.lo_dst[n] = a.lo_dst[n];
+      }
+      const int own = 32 - LaneSplit<N>::LH - (vu ? LaneSplit<N>::template rh_vu<MOM>() : LaneSplit<N>::rh_uv);
+      const long long strips = (d.ni() + own * N - 1) / (own * N);
+      // rows per warp: 64 (the four steps that fill the window cost 6%), halved while the grid would
+      // give fewer than 12 warps per SM
+      int rows = 64;
+      while (rows > 8 && strips * ((d.nj() + rows - 1) / rows) * nk < 148LL * 12) rows /= 2;
+      const dim3 blk(32, AW, 1), grd((unsigned)strips, (unsigned)((d.nj() + rows * AW - 1) / (rows * AW)), (unsigned)nk);
+      if (vu) k_adv_vu<R, S, REC, NF, N, LO, MOM><<<grd, blk, 0, s>>>(d, C, F, rows);
+      else k_adv_uv<R, S, REC, NF, N, LO, MOM><<<grd, blk, 0, s>>>(d, C, F, rows);
+      return (int)cudaGetLastError();
+    };
+    using std::integral_constant;
+    using F_ = std::false_type;
+    using T_ = std::true_type;
+    using I0 = integral_constant<int, 0>;
+    using I1 = integral_constant<int, 1>;
+    using I2_ = integral_constant<int, 2>;
+    auto with_n = [&](auto nn) -> int {
+      constexpr bool pairs = decltype(nn)::value <= 2;  // a tracer pair takes two cells per lane at most
+      if (a.mom == 1) return launch(I1(), nn, F_(), F_(), I1());
+      if (a.mom == 2) return launch(I1(), nn, F_(), F_(), I2_());
+      if (rec) return launch(I1(), nn, T_(), F_(), I0());
+      if constexpr (sizeof(R) == 4) {
+        if constexpr (pairs)
+          if (two && lo) return launch(I2_(), nn, F_(), T_(), I0());
+        if (lo) return launch(I1(), nn, F_(), T_(), I0());
+      }
+      if constexpr (pairs)
+        if (two) return launch(I2_(), nn, F_(), F_(), I0());
+      return launch(I1(), nn, F_(), F_(), I0());
+    };
+    if constexpr (sizeof(R) == 4) {
+      if (!two && aligned(4)) return with_n(integral_constant<int, 4>());
+      if (aligned(2)) return with_n(I2_());
+    }
+    return with_n(I1());
+  });
+}
+
 template <class R>
 int run_sweep_w2(const Dev& d, cudaStream_t s, R dt, R splitfac, int scheme, R* fa, R* fb, R* hi, const R* ww,
                  const int32_t* az, __half* lo_a, __half* lo_b) {
@@ -165,10 +249,10 @@ int run_sweep_w2(const Dev& d, cudaStream_t s, R dt, R splitfac, int scheme, R* 
 template <class R>
 int run_sweep_w(const Dev& d, cudaStream_t s, R dt, R splitfac, int scheme, int kshift, int itersmax,
                 const R* f, const R* fi_src, R* fi_dst, R* hi, R* adv, const R* ww, const int32_t* az,
-                unsigned long long* warn, uint8_t* code, __half* lo) {
+                unsigned long long* warn, uint8_t* code, __half* lo, int mom) {
   if (sizeof(R) == 8) lo = nullptr;
   if (itersmax > 1) {
-    if (code) return (int)cudaErrorInvalidValue;
+    if (code || mom) return (int)cudaErrorInvalidValue;
     dim3 blk(32, 2, 1);
     dim3 grd((d.ni() - 1 + blk.x - 1) / blk.x, (d.nj() - 1 + blk.y - 1) / blk.y, 1);
     k_sweep_w_iter<R><<<grd, blk, 0, s>>>(d, dt, splitfac, scheme, kshift, itersmax, f, fi_src, fi_dst, hi,
@@ -182,6 +266,12 @@ int run_sweep_w(const Dev& d, cudaStream_t s, R dt, R splitfac, int scheme, int 
     if (code)
       k_sweep_w<R, S, true><<<grd, blk, 0, s>>>(d, dt, splitfac, kshift, f, fi_src, fi_dst, hi, adv, ww, az, code,
                                                 lo);
+    else if (mom == 1)
+      k_sweep_w<R, S, false, 1><<<grd, blk, 0, s>>>(d, dt, splitfac, kshift, f, fi_src, fi_dst, hi, adv, ww, az,
+                                                    nullptr, lo);
+    else if (mom == 2)
+      k_sweep_w<R, S, false, 2><<<grd, blk, 0, s>>>(d, dt, splitfac, kshift, f, fi_src, fi_dst, hi, adv, ww, az,
+                                                    nullptr, lo);
     else
       k_sweep_w<R, S, false><<<grd, blk, 0, s>>>(d, dt, splitfac, kshift, f, fi_src, fi_dst, hi, adv, ww, az,
                                                  nullptr, lo);
@@ -276,7 +366,8 @@ template int run_sweep_w2<GB_REAL>(const Dev&, cudaStream_t, GB_REAL, GB_REAL, i
                                    const GB_REAL*, const int32_t*, __half*, __half*);
 template int run_sweep_w<GB_REAL>(const Dev&, cudaStream_t, GB_REAL, GB_REAL, int, int, int, const GB_REAL*,
                                   const GB_REAL*, GB_REAL*, GB_REAL*, GB_REAL*, const GB_REAL*, const int32_t*,
-                                  unsigned long long*, uint8_t*, __half*);
+                                  unsigned long long*, uint8_t*, __half*, int);
+template int run_adv_pass<GB_REAL>(const Dev&, cudaStream_t, bool, int, GB_REAL, int, GB_REAL, const AdvPass<GB_REAL>&);
 template int run_finalise<GB_REAL>(const Dev&, cudaStream_t, GB_REAL, GB_REAL*, const GB_REAL*, const GB_REAL*,
                                    const GB_REAL*, const uint8_t*);
 template int run_vdiff<GB_REAL>(const Dev&, cudaStream_t, GB_REAL, GB_REAL, GB_REAL, GB_REAL*, const GB_REAL*,

@@ -38,12 +38,40 @@ int run_sweep_h(const Dev& d, cudaStream_t s, int nk, R dt, R splitfac, int sche
                 const R* fi_src_b = nullptr, R* fi_dst_b = nullptr, __half* lo = nullptr,
                 __half* lo_b = nullptr, bool adv_init = false, bool du2d = false, bool di2d = false);
 
+// The two horizontal passes of a HALFSPLIT advection over nk levels (adv_fused.cuh), from level
+// pointers: vu false: u/2 then v/2; vu true: v/2 then u/2 (each sweep with splitfac 1/2). The fields
+// src, heights Di_src and carried errors lo_src are read, dst, Di_dst and lo_dst written: no array
+// may be both (cells are also read by warps that do not own them). adv: the flux-divergence sum,
+// started by the first pass (0 + its terms, in every cell) and added to by the second; may be null.
+// dst and Di_dst may be null in the second pass. src[1] != nullptr: a second tracer with the same
+// transports (then no adv and no codes). code_u, code_v: limiter branches (one tracer, no adv).
+// mom 1 / 2: the momentum advection of the U / V grid -- U, V are the 3D transports uu, vv, the first
+// pass takes no field (src[0] is not read) and advects uu (vv) over the height Di_src.
+// du2d, dv2d, di2d: DU, DV, Di_src are 2D arrays of values shared by every level.
+enum : int { ADV_FU = 1, ADV_PU = 2, ADV_FV = 4, ADV_PV = 8 };  // flux / update mask, u / v sweep
+template <class R>
+struct AdvPass {
+  const R* src[2] = {nullptr, nullptr};
+  R* dst[2] = {nullptr, nullptr};
+  const __half* lo_src[2] = {nullptr, nullptr};
+  __half* lo_dst[2] = {nullptr, nullptr};
+  const R *U = nullptr, *DU = nullptr, *V = nullptr, *DV = nullptr, *Di_src = nullptr;
+  R *Di_dst = nullptr, *adv = nullptr;
+  const uint8_t* flags = nullptr;  // the grid's masks, ADV_* bits of a byte per cell
+  uint8_t *code_u = nullptr, *code_v = nullptr;
+  int mom = 0;
+  bool du2d = false, dv2d = false, di2d = false;
+};
+template <class R>
+int run_adv_pass(const Dev& d, cudaStream_t s, bool vu, int nk, R dt, int scheme, R AH, const AdvPass<R>& a);
+
 // Vertical sweep on full 3D fields (level-0 pointers); code as above (face k stored at level k;
-// only without sub-iterations).
+// only without sub-iterations). mom 1 / 2 (no sub-iterations): ww is the vertical velocity of the T
+// points, the sweep uses its means at the U / V points (uv_advect_3d.F90:84,275; 0 at level 0).
 template <class R>
 int run_sweep_w(const Dev& d, cudaStream_t s, R dt, R splitfac, int scheme, int kshift, int itersmax,
                 const R* f, const R* fi_src, R* fi_dst, R* hi, R* adv, const R* ww, const int32_t* az,
-                unsigned long long* warn, uint8_t* code = nullptr, __half* lo = nullptr);
+                unsigned long long* warn, uint8_t* code = nullptr, __half* lo = nullptr, int mom = 0);
 
 // Depth-averaged momentum advection of one micro step with HALFSPLIT (adv2d_fused.cuh): UEx
 // (dir 0, U-grid masks) or VEx (dir 1, V-grid masks) from U, V, DU, DV in one launch, arithmetic
