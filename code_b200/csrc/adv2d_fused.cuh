@@ -18,10 +18,19 @@
 
 namespace gb {
 
-constexpr int FX = 56, FY = 16;             // own tile (region rows of two full warps)
-constexpr int RW = FX + 8, RH = FY + 4;     // staged region: i in [-4, FX+3], j in [-2, FY+1]
-constexpr int FTY = 8;                      // thread rows: a block is RW x FTY threads, lane x <-> region column
-constexpr int FT = RW * FTY;                // threads per block
+// launches of fewer large tiles than this take the small ones (two large tiles per SM)
+constexpr long long TILE2D_SMALL = 296;
+// A block of RW x FTY threads (lane x <-> region column) owns FX x FY cells of a staged region of
+// RW x RH, i in [-4, FX+3], j in [-2, FY+1]. Two sizes: 56 x 16 own cells (64 x 8 threads) where the
+// domain gives every SM work, 24 x 8 (32 x 4 threads, 1.7 times the halo) below, where the time is
+// the latency of one block: 128 x 96 FP64, both components 26 us in two launches of 21 large tiles,
+// 10 us in one launch of 156 small ones.
+template <int RW_, int FTY_>
+struct Tile2d {
+  static constexpr int RW = RW_, FTY = FTY_, FX = RW - 8, FY = 2 * FTY, RH = FY + 4, FT = RW * FTY;
+};
+using TileLarge = Tile2d<64, 8>;
+using TileSmall = Tile2d<32, 4>;
 
 // k*(a*s - b*s)*c as single rounded operations in this order: the volume and flux differences of
 // the cell updates. FP64: the plain operations (the FP64 build contracts nothing); FP32: explicit
@@ -37,8 +46,9 @@ __device__ __forceinline__ T add_r(T a, T b) {
   else return a + b;
 }
 
-template <class T>
+template <class T, class TL>
 struct Adv2dSmem {
+  static constexpr int RH = TL::RH, RW = TL::RW;
   T F0[RH][RW];   // advected quantity; reused for the field after the v sweep
   T F1[RH][RW];   // after the first u/2 sweep
   T Di[RH][RW];   // staged control-volume depth (the sweeps carry their rows' updated depths in registers)
@@ -48,19 +58,51 @@ struct Adv2dSmem {
   uint8_t mfu[RH][RW], mfv[RH][RW], mpu[RH][RW], mpv[RH][RW];
 };
 
+// The FP64 form of the log-law drag (bf_law_f32), the expressions of k_bottom_friction in its order.
+__device__ __forceinline__ void bf_law_f64(double zb, double zb0, double HH, double uloc, double vloc, double kappa,
+                                           double avmmol, int runtype, double& zn, double& rr, double& r) {
+  double x = kappa / log((zb + 0.5 * HH) / zb);
+  rr = x * x;
+  zn = zb;
+  if (runtype == 1) {
+    const double fricvel = sqrt(rr * (uloc * uloc + vloc * vloc));
+    zn = fmin(HH, zb0 + 0.1 * avmmol / fmax(avmmol, fricvel));
+    rr = (zn + 0.5 * HH) / zn;
+    x = kappa / log(rr);
+    rr = x * x;
+  }
+  r = rr * sqrt(uloc * uloc + vloc * vloc);
+}
+// velocity quotient, four-point mean and maximum of the bottom friction in its arithmetic
+template <class T, class TI>
+__device__ __forceinline__ T bf_quot(TI a, TI b) {
+  if constexpr (sizeof(T) == 4) return __fdividef(float(a), float(b));
+  else return a / b;
+}
+template <class T>
+__device__ __forceinline__ T bf_mean(T a, T b, T c, T e) {
+  if constexpr (sizeof(T) == 4) return __fmul_rn(0.25f, __fadd_rn(__fadd_rn(__fadd_rn(a, b), c), e));
+  else return 0.25 * (a + b + c + e);
+}
+template <class T>
+__device__ __forceinline__ T bf_max(T a, T b) {
+  if constexpr (sizeof(T) == 4) return fmaxf(a, b);
+  else return fmax(a, b);
+}
 
 // DIR 0: UEx on the U grid (fadv = U/DU, faces between U points); DIR 1: VEx on the V grid.
 // TI: the storage type of U, V, DU, DV and Ex (FP64 state arrays, or the FP32 working copies of
 // the mixed-precision micro step)
-template <class T, int S, int DIR, class TI>
+template <class TL, class T, int S, int DIR, class TI>
 __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __restrict__ U, const TI* __restrict__ V,
                                              const TI* __restrict__ DU, const TI* __restrict__ DV,
                                              const uint8_t* __restrict__ mflux_u,
                                              const uint8_t* __restrict__ mflux_v,
                                              const uint8_t* __restrict__ mupd_u, const uint8_t* __restrict__ mupd_v,
-                                             TI* __restrict__ Ex, const Bf2Args& bf) {
+                                             TI* __restrict__ Ex, const Bf2Args<TI>& bf) {
+  constexpr int FX = TL::FX, FY = TL::FY, RW = TL::RW, RH = TL::RH, FTY = TL::FTY;
   extern __shared__ unsigned char smem_raw[];
-  Adv2dSmem<T>& sm = *reinterpret_cast<Adv2dSmem<T>*>(smem_raw);
+  Adv2dSmem<T, TL>& sm = *reinterpret_cast<Adv2dSmem<T, TL>*>(smem_raw);
   const int ni = d.ni(), nj = d.nj();
   const long long sj = d.sj;
   const int ii0 = blockIdx.x * FX, jj0 = blockIdx.y * FY;
@@ -77,8 +119,7 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
     uint8_t a = 0, b = 0, c2 = 0, e2 = 0;
     if (iin && jj >= 0 && jj < nj) {
       const long long c = (long long)jj * sj + ii;
-      if constexpr (sizeof(T) == 4 && sizeof(TI) == 4)
-        if (bf.r) oq = DIR == 0 ? __fdividef(float(V[c]), float(DV[c])) : __fdividef(float(U[c]), float(DU[c]));
+      if (bf.r) oq = DIR == 0 ? bf_quot<T>(V[c], DV[c]) : bf_quot<T>(U[c], DU[c]);
       a = mflux_u[c];
       b = mflux_v[c];
       c2 = mupd_u[c];
@@ -115,7 +156,7 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
   // overlap by one column (warp 0: qc = 0..31, warp 1: qc = 31..62; warp 1's copy of column 31,
   // `dup`, updates and stores nothing), so that the left face flux of every cell a u sweep updates
   // is the flux of the lane before it (a warp shuffle, no shared-memory round trip or barrier).
-  // The own rows of a thread, r = 2 + ty + 8m (m = 0, 1), are the same in all three sweeps: their
+  // The own rows of a thread, r = 2 + ty + FTY*m (m = 0, 1), are the same in all three sweeps: their
   // depths and flux-divergence sums stay in registers.
   const int qc = q - (q >> 5);
   const bool dup = q == 32;
@@ -131,7 +172,7 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
       // the own rows, then the halo rows 0, 1, RH-2, RH-1 (thread rows 0..3)
-      const int r = m < 2 ? 2 + ty + 8 * m : (ty < 2 ? ty : RH - 4 + ty);
+      const int r = m < 2 ? 2 + ty + FTY * m : (ty < 2 ? ty : RH - 4 + ty);
       if (m == 2 && ty >= 4) continue;
       T fl = zero;
       if (fok)
@@ -175,7 +216,7 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
     if (col) {
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
-        const int r = 2 + ty + 8 * m;
+        const int r = 2 + ty + FTY * m;
         const int jj = jj0 - 2 + r;
         const T fio = sm.F1[r][qc];
         T fnew = fio;
@@ -198,7 +239,7 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
     const bool fok = qc >= 3 && qc <= RW - 5 && iic >= sub && iic <= ni - 2 - sub;
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
-      const int r = 2 + ty + 8 * m;
+      const int r = 2 + ty + FTY * m;
       T fl = zero;
       if (fok)
         fl = face_flux_s<T, S>(sm.Ua[r][qc], sm.DUa[r][qc], sm.F0[r][qc - 1], sm.F0[r][qc], sm.F0[r][qc + 1],
@@ -216,140 +257,91 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
       }
     }
   }
-  if constexpr (sizeof(T) == 4 && sizeof(TI) == 4) {
-    if (bf.r && qown) {
+  // ---- the bottom friction of the own points (bottom_friction.F90:48-150)
+  if (bf.r && qown) {
 #pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        const int r = 2 + ty + 8 * m;
-        const int jj = jj0 - 2 + r;
-        if (iic >= ni || jj >= nj) continue;
-        const long long c = (long long)jj * sj + iic;
-        const int i = iic + d.imin - HALO, j = jj + d.jmin - HALO;
-        const bool in = i >= d.imin && i <= d.imax && j >= d.jmin && j <= d.jmax;
-        const float q4 = 0.25f;
-        float uloc, vloc, HHl;
-        bool on;
-        if (DIR == 0) {
-          on = i <= d.imax + HALO - 1 && bf.mask[c] > 0;
-          if (!on) continue;
-          vloc = in ? __fmul_rn(q4, __fadd_rn(__fadd_rn(__fadd_rn(sm.Q[r][qc], sm.Q[r][qc + 1]), sm.Q[r - 1][qc]),
-                                              sm.Q[r - 1][qc + 1]))
-                    : 0.f;
-          uloc = __fdividef(float(U[c]), float(DU[c]));
-          HHl = fmaxf(bf.min_depth, float(DU[c]));
-        } else {
-          on = j <= d.jmax + HALO - 1 && bf.mask[c] > 0;
-          if (!on) continue;
-          if (in)
-            uloc = __fmul_rn(q4, __fadd_rn(__fadd_rn(__fadd_rn(sm.Q[r][qc], sm.Q[r][qc - 1]), sm.Q[r + 1][qc]),
-                                           sm.Q[r + 1][qc - 1]));
-          else
-            uloc = (i <= d.imax + HALO - 1 && bf.au[c] > 0) ? sm.Q[r][qc] : 0.f;
-          vloc = __fdividef(float(V[c]), float(DV[c]));
-          HHl = fmaxf(bf.min_depth, float(DV[c]));
-        }
-        const BfLaw b = bf_law_f32(bf.zb[c], bf.zb0[c], HHl, uloc, vloc, bf.kappa, bf.avmmol, bf.runtype);
-        if (bf.runtype == 1) bf.zb[c] = b.zn;
-        bf.rr[c] = b.rr;
-        bf.r[c] = b.r;
+    for (int m = 0; m < 2; ++m) {
+      const int r = 2 + ty + FTY * m;
+      const int jj = jj0 - 2 + r;
+      if (iic >= ni || jj >= nj) continue;
+      const long long c = (long long)jj * sj + iic;
+      const int i = iic + d.imin - HALO, j = jj + d.jmin - HALO;
+      const bool in = i >= d.imin && i <= d.imax && j >= d.jmin && j <= d.jmax;
+      T uloc, vloc, HHl;
+      if (DIR == 0) {
+        if (!(i <= d.imax + HALO - 1 && bf.mask_at(c) > 0)) continue;
+        vloc = in ? bf_mean<T>(sm.Q[r][qc], sm.Q[r][qc + 1], sm.Q[r - 1][qc], sm.Q[r - 1][qc + 1]) : zero;
+        uloc = bf_quot<T>(U[c], DU[c]);
+        HHl = bf_max<T>(T(bf.min_depth), T(DU[c]));
+      } else {
+        if (!(j <= d.jmax + HALO - 1 && bf.mask_at(c) > 0)) continue;
+        if (in)
+          uloc = bf_mean<T>(sm.Q[r][qc], sm.Q[r][qc - 1], sm.Q[r + 1][qc], sm.Q[r + 1][qc - 1]);
+        else
+          uloc = (i <= d.imax + HALO - 1 && bf.au_at(c) > 0) ? sm.Q[r][qc] : zero;
+        vloc = bf_quot<T>(V[c], DV[c]);
+        HHl = bf_max<T>(T(bf.min_depth), T(DV[c]));
       }
+      T zn, rr, rv;
+      if constexpr (sizeof(T) == 4) {
+        const BfLaw b = bf_law_f32(float(bf.zb[c]), float(bf.zb0[c]), HHl, uloc, vloc, float(bf.kappa), float(bf.avmmol),
+                                   bf.runtype);
+        zn = b.zn;
+        rr = b.rr;
+        rv = b.r;
+      } else {
+        bf_law_f64(bf.zb[c], bf.zb0 ? bf.zb0[c] : 0.0, HHl, uloc, vloc, bf.kappa, bf.avmmol, bf.runtype, zn, rr, rv);
+      }
+      if (bf.runtype == 1) bf.zb[c] = (TI)zn;
+      bf.rr[c] = (TI)rr;
+      bf.r[c] = (TI)rv;
     }
   }
 }
 
-template <class T, int S, int DIR, class TI>
-__global__ void __launch_bounds__(FT) k_uvadv2d_fused(Dev d, T dt, const TI* __restrict__ U,
-                                                      const TI* __restrict__ V, const TI* __restrict__ DU,
-                                                      const TI* __restrict__ DV,
-                                                      const uint8_t* __restrict__ mflux_u,
-                                                      const uint8_t* __restrict__ mflux_v,
-                                                      const uint8_t* __restrict__ mupd_u,
-                                                      const uint8_t* __restrict__ mupd_v, TI* __restrict__ Ex,
-                                                      Bf2Args bf) {
-  uvadv2d_tile<T, S, DIR, TI>(d, dt, U, V, DU, DV, mflux_u, mflux_v, mupd_u, mupd_v, Ex, bf);
-}
-
-// Both components in one launch (blockIdx.z = 0: UEx on the U grid, 1: VEx on the V grid): the
-// same tiles as two k_uvadv2d_fused launches, one grid, one tail. Four blocks per SM (32 registers,
-// no spills; the shared memory holds four): the issue-bound sweeps then have 64 warps to choose
-// from instead of 48.
+// Both components in one launch (blockIdx.z = 0: UEx on the U grid, 1: VEx on the V grid): one grid,
+// one tail. FP32 working copies: 2048 threads per SM (32 registers, no spills; the shared memory holds
+// them): the issue-bound sweeps then have 64 warps to choose from instead of 48. FP64 arrays: 1024.
 struct Adv2dMasks {
   const uint8_t *mflux_u, *mflux_v, *mupd_u, *mupd_v;
 };
-template <class T, int S, class TI>
-__global__ void __launch_bounds__(FT, 4) k_uvadv2d_both(Dev d, T dt, const TI* __restrict__ U, const TI* __restrict__ V,
-                                                     const TI* __restrict__ DU, const TI* __restrict__ DV,
-                                                     Adv2dMasks mu, Adv2dMasks mv, TI* __restrict__ UEx,
-                                                     TI* __restrict__ VEx, Bf2Args bfu, Bf2Args bfv) {
+template <class TL, class T, int S, class TI>
+__global__ void __launch_bounds__(TL::FT, (sizeof(TI) == 4 ? 2048 : 1024) / TL::FT)
+    k_uvadv2d_both(Dev d, T dt, const TI* __restrict__ U, const TI* __restrict__ V, const TI* __restrict__ DU,
+                   const TI* __restrict__ DV, Adv2dMasks mu, Adv2dMasks mv, TI* __restrict__ UEx, TI* __restrict__ VEx,
+                   Bf2Args<TI> bfu, Bf2Args<TI> bfv) {
   if (blockIdx.z == 0)
-    uvadv2d_tile<T, S, 0, TI>(d, dt, U, V, DU, DV, mu.mflux_u, mu.mflux_v, mu.mupd_u, mu.mupd_v, UEx, bfu);
+    uvadv2d_tile<TL, T, S, 0, TI>(d, dt, U, V, DU, DV, mu.mflux_u, mu.mflux_v, mu.mupd_u, mu.mupd_v, UEx, bfu);
   else
-    uvadv2d_tile<T, S, 1, TI>(d, dt, U, V, DU, DV, mv.mflux_u, mv.mflux_v, mv.mupd_u, mv.mupd_v, VEx, bfv);
+    uvadv2d_tile<TL, T, S, 1, TI>(d, dt, U, V, DU, DV, mv.mflux_u, mv.mflux_v, mv.mupd_u, mv.mupd_v, VEx, bfv);
 }
 
-template <class T, int S, int DIR, class TI>
-int launch_uvadv2d_fused(const Dev& d, cudaStream_t s, T dt, const TI* U, const TI* V, const TI* DU, const TI* DV,
-                         const uint8_t* mflux_u, const uint8_t* mflux_v, const uint8_t* mupd_u,
-                         const uint8_t* mupd_v, TI* Ex, const Bf2Args& bf) {
-  const size_t smem = sizeof(Adv2dSmem<T>);
-  // opt-in above 48 KB of shared memory (a host-side setting of the current device's function)
-  const cudaError_t e = cudaFuncSetAttribute(k_uvadv2d_fused<T, S, DIR, TI>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return (int)e;
-  dim3 grd((d.ni() + FX - 1) / FX, (d.nj() + FY - 1) / FY, 1);
-  k_uvadv2d_fused<T, S, DIR, TI><<<grd, dim3(RW, FTY, 1), smem, s>>>(d, dt, U, V, DU, DV, mflux_u, mflux_v, mupd_u,
-                                                                      mupd_v, Ex, bf);
-  return (int)cudaGetLastError();
-}
-
+// T: arithmetic, TI: the 2D fields (FP64 state arrays or FP32 working copies)
 template <class T, class TI>
-int run_uvadv2d_fused_t(const Dev& d, cudaStream_t s, int dir, T dt, int scheme, const TI* U, const TI* V,
-                        const TI* DU, const TI* DV, const uint8_t* mflux_u, const uint8_t* mflux_v,
-                        const uint8_t* mupd_u, const uint8_t* mupd_v, TI* Ex, const Bf2Args& bf) {
+int run_uvadv2d(const Dev& d, cudaStream_t s, T dt, int scheme, const TI* U, const TI* V, const TI* DU, const TI* DV,
+                const uint8_t* const* mu, const uint8_t* const* mv, TI* UEx, TI* VEx, const Bf2Args<TI>* bfu,
+                const Bf2Args<TI>* bfv) {
   return dispatch_scheme(scheme, [&](auto sc) {
     constexpr int S = decltype(sc)::value;
-    return dir == 0
-               ? launch_uvadv2d_fused<T, S, 0, TI>(d, s, dt, U, V, DU, DV, mflux_u, mflux_v, mupd_u, mupd_v, Ex, bf)
-               : launch_uvadv2d_fused<T, S, 1, TI>(d, s, dt, U, V, DU, DV, mflux_u, mflux_v, mupd_u, mupd_v, Ex, bf);
+    auto go = [&](auto tile) -> int {
+      using TL = decltype(tile);
+      auto kern = k_uvadv2d_both<TL, T, S, TI>;
+      const size_t smem = sizeof(Adv2dSmem<T, TL>);
+      if (smem > 48 * 1024) {  // opt-in (a host-side setting of the current device's function)
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+      }
+      const dim3 grd((d.ni() + TL::FX - 1) / TL::FX, (d.nj() + TL::FY - 1) / TL::FY, 2);
+      kern<<<grd, dim3(TL::RW, TL::FTY, 1), smem, s>>>(
+          d, dt, U, V, DU, DV, Adv2dMasks{mu[0], mu[1], mu[2], mu[3]}, Adv2dMasks{mv[0], mv[1], mv[2], mv[3]}, UEx, VEx,
+          bfu ? *bfu : Bf2Args<TI>{}, bfv ? *bfv : Bf2Args<TI>{});
+      return (int)cudaGetLastError();
+    };
+    const long long large = 2LL * ((d.ni() + TileLarge::FX - 1) / TileLarge::FX) *
+                            ((d.nj() + TileLarge::FY - 1) / TileLarge::FY);
+    if (large < TILE2D_SMALL) return go(TileSmall());
+    return go(TileLarge());
   });
 }
-
-template <class T>
-int run_uvadv2d_fused(const Dev& d, cudaStream_t s, int dir, T dt, int scheme, const double* U, const double* V,
-                      const double* DU, const double* DV, const uint8_t* mflux_u, const uint8_t* mflux_v,
-                      const uint8_t* mupd_u, const uint8_t* mupd_v, double* Ex) {
-  return run_uvadv2d_fused_t<T, double>(d, s, dir, dt, scheme, U, V, DU, DV, mflux_u, mflux_v, mupd_u, mupd_v, Ex,
-                                        Bf2Args{});
-}
-
-// FP32 arithmetic on the FP32 working copies of the mixed-precision micro step (defined in the
-// FP32 translation unit only)
-#if defined(GB_REAL_IS_FLOAT)
-
-int run_uvadv2d_fused_f32(const Dev& d, cudaStream_t s, int dir, float dt, int scheme, const float* U,
-                          const float* V, const float* DU, const float* DV, const uint8_t* mflux_u,
-                          const uint8_t* mflux_v, const uint8_t* mupd_u, const uint8_t* mupd_v, float* Ex,
-                          const Bf2Args* bf) {
-  return run_uvadv2d_fused_t<float, float>(d, s, dir, dt, scheme, U, V, DU, DV, mflux_u, mflux_v, mupd_u, mupd_v,
-                                           Ex, bf ? *bf : Bf2Args{});
-}
-
-int run_uvadv2d_both_f32(const Dev& d, cudaStream_t s, float dt, int scheme, const float* U, const float* V,
-                         const float* DU, const float* DV, const uint8_t* const* mu, const uint8_t* const* mv,
-                         float* UEx, float* VEx, const Bf2Args* bfu, const Bf2Args* bfv) {
-  return dispatch_scheme(scheme, [&](auto sc) {
-    constexpr int S = decltype(sc)::value;
-    const size_t smem = sizeof(Adv2dSmem<float>);
-    const cudaError_t e = cudaFuncSetAttribute(k_uvadv2d_both<float, S, float>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    dim3 grd((d.ni() + FX - 1) / FX, (d.nj() + FY - 1) / FY, 2);
-    k_uvadv2d_both<float, S, float><<<grd, dim3(RW, FTY, 1), smem, s>>>(
-        d, dt, U, V, DU, DV, Adv2dMasks{mu[0], mu[1], mu[2], mu[3]}, Adv2dMasks{mv[0], mv[1], mv[2], mv[3]}, UEx,
-        VEx, bfu ? *bfu : Bf2Args{}, bfv ? *bfv : Bf2Args{});
-    return (int)cudaGetLastError();
-  });
-}
-#endif
 
 }  // namespace gb

@@ -554,11 +554,11 @@ __global__ void k_depth_update(Dev d, Bc2 s, Bc2W w) {
   if (av(i, j) > 0) dry_v(i, j) = fmax(0.0, fmin(1.0, (DV_(i, j) - d1) * d2i));
 }
 
-// k_accum_sealevel and k_depth_update as one launch, for the micro-step loop without open
-// boundaries. The elevations ping-pong between the state's z and zo arrays: s.f2[Z] holds the
-// elevations before the step and is only read; the new ones go to s.f2[ZO], so the old array is
-// exactly the reference's zo = z of sealevel.F90:89 and the caller swaps the two pointers after
-// the launch. The depths of a U (V) point need the new elevation of the next T point, which the
+// k_accum_sealevel and k_depth_update as one launch, for the micro-step loop (open boundaries: after
+// update_2d_bdy has set their elevations in z). The elevations ping-pong between the state's z and
+// zo arrays: s.f2[Z] holds the elevations before the step and is only read; the new ones go to
+// s.f2[ZO], so the old array is exactly the reference's zo = z of sealevel.F90:89 and the caller
+// swaps the two pointers after the launch. The depths of a U (V) point need the new elevation of the next T point, which the
 // thread forms itself from the same inputs with the same expression (no thread reads a value
 // that another writes). Same values as the two kernels, bit for bit. flags: bit 0 accumulates
 // Uint/Vint; bit 1 writes the drying factor dry_z, which no micro-step kernel reads: the caller asks
@@ -1194,9 +1194,50 @@ int do_adv2d(getm_ctx* ctx, T dt, T* f, const T* U, const T* V, const T* DUa, co
 // uv_advect.F90:94-300 on (U, V, DU, DV) -> UEx, VEx (split schemes). The plain step works in
 // FP64 (bit for bit with the reference); the mixed step advects the depth-averaged momentum in
 // FP32 and widens the increments into the FP64 UEx / VEx.
+// Arguments of the bottom friction formed with the momentum advection (Bf2Args), for the FP64 state
+// arrays (w null) or the FP32 working copies.
+template <class TI>
+void bf2_args(const getm_bc_state* st, const Bc2W* w, Bf2Args<TI> (&bf)[2]) {
+  for (int dir = 0; dir < 2; ++dir) {
+    auto f = [&](int q) -> TI* {
+      if constexpr (sizeof(TI) == 4) return w->w[q];
+      else return st->f2[q];
+    };
+    Bf2Args<TI>& b = bf[dir];
+    if constexpr (sizeof(TI) == 4) {
+      b.mask8 = w->m8[dir == 0 ? 1 : 2];
+      b.au8 = w->m8[1];
+    } else {
+      b.mask32 = dir == 0 ? st->au : st->av;
+      b.au32 = st->au;
+    }
+    b.zb = f(dir == 0 ? ZUB : ZVB);
+    b.zb0 = f(dir == 0 ? ZUB0 : ZVB0);
+    b.r = f(dir == 0 ? RU : RV);
+    b.rr = f(dir == 0 ? RUU : RVV);
+    b.kappa = st->par[P_KAPPA];
+    b.avmmol = st->par[P_AVMMOL];
+    b.min_depth = st->par[P_MIN_DEPTH];
+    b.runtype = st->ipar[I_RUNTYPE];
+  }
+}
+
+// the U (dir 0) and V grid's masks of the 2D advection: flux-u, flux-v, update-u, update-v
+void adv2d_masks(const getm_ctx* ctx, const uint8_t* (&m)[2][4]) {
+  for (int dir = 0; dir < 2; ++dir) {
+    getm_adv_grid g;
+    grid_for_tag(ctx, dir == 0 ? GETM_U_TAG : GETM_V_TAG, &g);
+    m[dir][0] = g.mask_uflux;
+    m[dir][1] = g.mask_vflux;
+    m[dir][2] = g.mask_uupdate;
+    m[dir][3] = g.mask_vupdate;
+  }
+}
+
+// bf: with HALFSPLIT, also form the bottom friction (of U, V, DU_, DV_ = the state's fields)
 template <class T>
 int uv_advect_2d_t(getm_ctx* ctx, const getm_bc_state* st, const double* U, const double* V, const double* DU_,
-                   const double* DV_) {
+                   const double* DV_, bool bf) {
   const Dev& d = ctx->dev;
   cudaStream_t s = ctx->stream;
   const long long n2 = n2d(d);
@@ -1208,14 +1249,14 @@ int uv_advect_2d_t(getm_ctx* ctx, const getm_bc_state* st, const double* U, cons
     return GETM_OK;
   }
   if (split == GETM_HALFSPLIT && is_split_scheme(hor)) {
-    // all three sweeps of each component in one launch (adv2d_fused.cuh)
-    for (int dir = 0; dir < 2; ++dir) {
-      getm_adv_grid g;
-      grid_for_tag(ctx, dir == 0 ? GETM_U_TAG : GETM_V_TAG, &g);
-      GB_TIMED(GETM_TIM_BC2D, run_uvadv2d_fused<T>(d, s, dir, T(st->par[P_DTM]), hor, U, V, DU_, DV_, g.mask_uflux,
-                                                   g.mask_vflux, g.mask_uupdate, g.mask_vupdate, Ex[dir]),
-               "uv_advect");
-    }
+    // all three sweeps of both components in one launch (adv2d_fused.cuh)
+    const uint8_t* masks[2][4];
+    adv2d_masks(ctx, masks);
+    Bf2Args<double> b[2];
+    if (bf) bf2_args<double>(st, nullptr, b);
+    GB_TIMED(GETM_TIM_BC2D, (run_uvadv2d<T, double>(d, s, T(st->par[P_DTM]), hor, U, V, DU_, DV_, masks[0], masks[1],
+                                                    Ex[0], Ex[1], &b[0], &b[1])),
+             "uv_advect");
     return GETM_OK;
   }
   // 2D scratch (NB2 FP64-sized arrays) viewed as T
@@ -1249,9 +1290,9 @@ int uv_advect_2d_t(getm_ctx* ctx, const getm_bc_state* st, const double* U, cons
 }
 
 int uv_advect_2d(getm_ctx* ctx, const getm_bc_state* st, const double* U, const double* V, const double* DU_,
-                 const double* DV_) {
-  return st->prec3d == 8 ? uv_advect_2d_t<double>(ctx, st, U, V, DU_, DV_)
-                         : uv_advect_2d_t<float>(ctx, st, U, V, DU_, DV_);
+                 const double* DV_, bool bf = false) {
+  return st->prec3d == 8 ? uv_advect_2d_t<double>(ctx, st, U, V, DU_, DV_, bf)
+                         : uv_advect_2d_t<float>(ctx, st, U, V, DU_, DV_, bf);
 }
 
 #define GB_K2(kernel, ...)                                         \
@@ -1328,9 +1369,9 @@ bool pairs_ok(const Dev& d, const Bc2& s, const Bc2W& w) {
 // velocity (:193-216, :356-379). Mixed micro step (wp): the update on the working copies, with
 // the term it needs formed in the same launch when `cor` (see integrate_2d).
 template <int DIR>
-// fused (the FP64 micro-step loop without open boundaries; always for the mixed step): the update
-// forms the Coriolis term it needs itself when `cor`, and the term of the other velocity is left to
-// the next update (or to the end of the loop) instead of a k_coriolis launch after each update.
+// fused (the micro-step loop; always for the mixed step): the update forms the Coriolis term it needs
+// itself when `cor`, and the term of the other velocity is left to the next update (or to the end of
+// the loop) instead of a k_coriolis launch after each update.
 int momentum_2d(getm_ctx* ctx, const getm_bc_state* st, const Bc2W* wp, bool cor, bool fused = false) {
   const Dev& d = ctx->dev;
   const Bc2 s = to_bc2(st);
@@ -1349,9 +1390,10 @@ int momentum_2d(getm_ctx* ctx, const getm_bc_state* st, const Bc2W* wp, bool cor
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, (int)e, DIR == 0 ? "umomentum" : "vmomentum");
   }
-  if (wp || fused) return GETM_OK;
+  if (wp) return GETM_OK;
   int r;
   if ((r = mirror_bdy<double>(ctx, st->f2[DIR == 0 ? U_ : V_], DIR, 1))) return r;
+  if (fused) return GETM_OK;
   TimerScope ts(ctx, GETM_TIM_BC2D);
   k_coriolis<DIR, false><<<grid2(d), kBlk2, 0, cs>>>(d, s, w);
   const cudaError_t e = cudaGetLastError();
@@ -1359,7 +1401,7 @@ int momentum_2d(getm_ctx* ctx, const getm_bc_state* st, const Bc2W* wp, bool cor
 }
 
 // m2d.F90:412-490 integrate_2d (closed boundaries; no residual; Am <= 0, An_method = 0)
-// zswap (the micro-step loop without open boundaries): sealevel and depth_update as one launch that
+// zswap (the micro-step loop): sealevel and depth_update as one launch that
 // writes the new elevations into st->f2[ZO]; the caller then swaps st->f2[Z] and st->f2[ZO]. With
 // zswap, dryz = false leaves dry_z as it is (a micro step that neither a macro step nor the
 // caller follows).
@@ -1378,10 +1420,11 @@ int integrate_2d(getm_ctx* ctx, getm_bc_state* st, int loop, const Bc2W* wp = nu
   };
   int rc = GETM_OK;
   const bool bf_due = (loop - 1) % ip[I_MM] == 0;
-  // the mixed micro step forms the bottom friction inside its momentum-advection kernels (they
-  // stage the same velocities); the separate kernel otherwise (and with the fused micro-step
-  // kernels switched off, for the comparison of the two forms)
-  const bool bf_fused = mix && bf_due && ip[I_VEL2D_HOR] != NOADV && fused_micro_enabled();
+  // the micro step forms the bottom friction inside its momentum-advection launch (which stages the
+  // same velocities) where that is the fused one; the separate kernel otherwise (and with the fused
+  // micro-step kernels switched off, for the comparison of the two forms)
+  const bool bf_fused = bf_due && fused_micro_enabled() && ip[I_VEL2D_HOR] != NOADV &&
+                        (mix || (ip[I_VEL2D_SPLIT] == GETM_HALFSPLIT && is_split_scheme(ip[I_VEL2D_HOR])));
   if (bf_due && !bf_fused && (rc = bottom_friction_2d(ctx, st, ip[I_RUNTYPE], wp))) return rc;
   if (mix) {
     const int hor = ip[I_VEL2D_HOR];
@@ -1391,35 +1434,16 @@ int integrate_2d(getm_ctx* ctx, getm_bc_state* st, int loop, const Bc2W* wp = nu
     } else {
       // both components in one launch: UEx and VEx each read U, V, DU, DV only
       const uint8_t* masks[2][4];
-      Bf2Args bf[2]{};
-      for (int dir = 0; dir < 2; ++dir) {
-        getm_adv_grid g;
-        grid_for_tag(ctx, dir == 0 ? GETM_U_TAG : GETM_V_TAG, &g);
-        masks[dir][0] = g.mask_uflux;
-        masks[dir][1] = g.mask_vflux;
-        masks[dir][2] = g.mask_uupdate;
-        masks[dir][3] = g.mask_vupdate;
-        if (bf_fused) {
-          bf[dir].mask = w.m8[dir == 0 ? 1 : 2];
-          bf[dir].au = w.m8[1];
-          bf[dir].zb = w.w[dir == 0 ? ZUB : ZVB];
-          bf[dir].zb0 = w.w[dir == 0 ? ZUB0 : ZVB0];
-          bf[dir].r = w.w[dir == 0 ? RU : RV];
-          bf[dir].rr = w.w[dir == 0 ? RUU : RVV];
-          bf[dir].kappa = float(st->par[P_KAPPA]);
-          bf[dir].avmmol = float(st->par[P_AVMMOL]);
-          bf[dir].min_depth = float(st->par[P_MIN_DEPTH]);
-          bf[dir].runtype = ip[I_RUNTYPE];
-        }
-      }
+      adv2d_masks(ctx, masks);
+      Bf2Args<float> bf[2];
+      if (bf_fused) bf2_args<float>(st, &w, bf);
       GB_TIMED(GETM_TIM_BC2D,
-               run_uvadv2d_both_f32(d, ctx->stream, float(st->par[P_DTM]), hor, w.w[U_], w.w[V_], w.w[DU], w.w[DV],
-                                    masks[0], masks[1], w.w[UEX], w.w[VEX], bf_fused ? &bf[0] : nullptr,
-                                    bf_fused ? &bf[1] : nullptr),
+               (run_uvadv2d<float, float>(d, ctx->stream, float(st->par[P_DTM]), hor, w.w[U_], w.w[V_], w.w[DU], w.w[DV],
+                                          masks[0], masks[1], w.w[UEX], w.w[VEX], &bf[0], &bf[1])),
                "uv_advect");
     }
   } else {
-    rc = uv_advect_2d(ctx, st, st->f2[U_], st->f2[V_], st->f2[DU], st->f2[DV]);
+    rc = uv_advect_2d(ctx, st, st->f2[U_], st->f2[V_], st->f2[DU], st->f2[DV], bf_fused);
     if (rc) return rc;
   }
   // umomentum / vmomentum: transport update, mirror_bdy_2d (momentum.F90:190,353), Coriolis term.
@@ -1428,7 +1452,7 @@ int integrate_2d(getm_ctx* ctx, getm_bc_state* st, int loop, const Bc2W* wp = nu
   // it gives the same value. The first update of a getm_time_loop call (first) reads the stored
   // term instead -- the state's fU/fV, which need not match the velocities (a start from rest of
   // the Coriolis terms) -- and getm_time_loop forms the term of the last update at its end.
-  // the FP64 loop without open boundaries forms the Coriolis terms like the mixed step (zswap)
+  // the FP64 loop forms the Coriolis terms like the mixed step (zswap)
   auto umom = [&](bool cor) -> int { return momentum_2d<0>(ctx, st, wp, cor, zswap); };
   auto vmom = [&](bool cor) -> int { return momentum_2d<1>(ctx, st, wp, cor, zswap); };
   if (ip[I_UFIRST2D]) {
@@ -1440,8 +1464,8 @@ int integrate_2d(getm_ctx* ctx, getm_bc_state* st, int loop, const Bc2W* wp = nu
   }
   // update_2d_bdy sets the boundary elevations after the Uint accumulation and before sealevel
   // (m2d.F90:467-476); the accumulation does not touch z, so it runs inside the sealevel kernel
+  if (!mix && (rc = bdy_2d(ctx, s, loop))) return rc;
   if (zswap) {
-    if (ctx->has_bdy) return fail(ctx, GETM_ERR_STATE, "integrate_2d: fused sealevel with open boundaries");
     const int flags = (ip[I_RUNTYPE] > 1 ? 1 : 0) | (dryz ? 2 : 0);
     if (mix && pairs_ok(d, s, w)) {
       TimerScope ts(ctx, GETM_TIM_BC2D);
@@ -1454,7 +1478,6 @@ int integrate_2d(getm_ctx* ctx, getm_bc_state* st, int loop, const Bc2W* wp = nu
     std::swap(st->f2[Z], st->f2[ZO]);
     return nan_sweep_due(ctx, st, loop);
   }
-  if (!mix && (rc = bdy_2d(ctx, s, loop))) return rc;
   rc = mix ? k2(k_accum_sealevel<true>, d, s, w, ip[I_RUNTYPE] > 1 ? 1 : 0)
            : k2(k_accum_sealevel<false>, d, s, w, ip[I_RUNTYPE] > 1 ? 1 : 0);
   if (rc) return cuda_fail(ctx, rc, "sealevel");
@@ -2130,11 +2153,10 @@ int getm_time_loop(getm_ctx* ctx, getm_bc_state* st_user, int n0, int count) {
   int rc = check_state(ctx, st_user);
   if (rc) return rc;
   if ((rc = ensure_bc_scratch(ctx, (size_t)st_user->prec3d))) return rc;
-  // Without open boundaries the micro steps update the elevations by pointer ping-pong between z
-  // and zo (k_sealevel_depth) on a copy of the state table; after an odd number of swaps the two
-  // arrays' contents are exchanged at the end, so the caller's z and zo hold what the reference's
-  // would. The integer settings the steps update (ufirst2d/3d, nan_warned) are copied back.
-  const bool zswap = !ctx->has_bdy && fused_micro_enabled();
+  // The micro steps update the elevations by pointer ping-pong between z and zo (k_sealevel_depth) on
+  // a copy of the state table; after an odd number of swaps the two arrays' contents are exchanged at
+  // the end, so the caller's z and zo hold what the reference's would. The integer settings the steps update (ufirst2d/3d, nan_warned) are copied back.
+  const bool zswap = fused_micro_enabled();
   getm_bc_state loc = *st_user;
   rc = time_loop(ctx, zswap ? &loc : st_user, n0, count, zswap);
   if (zswap) {

@@ -388,9 +388,14 @@ template int run_check_range<GB_REAL>(const Dev&, cudaStream_t, const GB_REAL*, 
 // ---- fused 2D momentum advection ----
 #include "adv2d_fused.cuh"
 namespace gb {
-template int run_uvadv2d_fused<GB_REAL>(const Dev&, cudaStream_t, int, GB_REAL, int, const double*, const double*,
-                                        const double*, const double*, const uint8_t*, const uint8_t*,
-                                        const uint8_t*, const uint8_t*, double*);
+template int run_uvadv2d<GB_REAL, double>(const Dev&, cudaStream_t, GB_REAL, int, const double*, const double*,
+                                          const double*, const double*, const uint8_t* const*, const uint8_t* const*,
+                                          double*, double*, const Bf2Args<double>*, const Bf2Args<double>*);
+#if defined(GB_REAL_IS_FLOAT)
+template int run_uvadv2d<float, float>(const Dev&, cudaStream_t, float, int, const float*, const float*, const float*,
+                                       const float*, const uint8_t* const*, const uint8_t* const*, float*, float*,
+                                       const Bf2Args<float>*, const Bf2Args<float>*);
+#endif
 }  // namespace gb
 
 // ---- adjoint of the tracer step ----

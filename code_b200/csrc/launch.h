@@ -73,37 +73,29 @@ int run_sweep_w(const Dev& d, cudaStream_t s, R dt, R splitfac, int scheme, int 
                 const R* f, const R* fi_src, R* fi_dst, R* hi, R* adv, const R* ww, const int32_t* az,
                 unsigned long long* warn, uint8_t* code = nullptr, __half* lo = nullptr, int mom = 0);
 
-// Depth-averaged momentum advection of one micro step with HALFSPLIT (adv2d_fused.cuh): UEx
-// (dir 0, U-grid masks) or VEx (dir 1, V-grid masks) from U, V, DU, DV in one launch, arithmetic
-// in T; Ex is FP64.
-template <class T>
-int run_uvadv2d_fused(const Dev& d, cudaStream_t s, int dir, T dt, int scheme, const double* U, const double* V,
-                      const double* DU, const double* DV, const uint8_t* mflux_u, const uint8_t* mflux_v,
-                      const uint8_t* mupd_u, const uint8_t* mupd_v, double* Ex);
-// The bottom friction of the micro step (bottom_friction.F90:48-150), formed by the momentum
-// advection kernel of the same component from the velocities it stages anyway: DIR 0 the U points
-// (ru, ruu; zub for runtype 1), DIR 1 the V points (rv, rvv; zvb). FP32 arithmetic, the operations
-// of k_bottom_friction_f32t (bc.cu) in the same order, so the same values. r == nullptr: off.
+// Depth-averaged momentum advection of one micro step with HALFSPLIT (adv2d_fused.cuh): UEx and VEx
+// from U, V, DU, DV in one launch, arithmetic in T on fields of type TI. With bfu, bfv also the bottom
+// friction of the micro step (bottom_friction.F90:48-150), from the velocities the tiles stage
+// anyway: bfu the U points (ru, ruu; zub for runtype 1), bfv the V points (rv, rvv; zvb) -- the
+// operations of the separate bottom-friction kernels (bc.cu) in the same order, so the same values.
+// r == nullptr: off. The masks are int32 state arrays or (FP32 working copies) their uint8 copies.
+template <class TI>
 struct Bf2Args {
-  const uint8_t* mask;  // au (DIR 0) / av (DIR 1), uint8 copies
-  const uint8_t* au;    // DIR 1: the U points' mask for the velocity outside the interior
-  float* zb;            // zub / zvb (FP32 working copies)
-  const float* zb0;     // zub0 / zvb0
-  float* r;             // ru / rv (FP32 working copies)
-  float* rr;            // ruu / rvv
-  float kappa, avmmol, min_depth;
-  int runtype;
+  const int32_t *mask32 = nullptr, *au32 = nullptr;
+  const uint8_t *mask8 = nullptr, *au8 = nullptr;  // the component's mask; the U points' mask
+  TI* zb = nullptr;                                // zub / zvb
+  const TI* zb0 = nullptr;                         // zub0 / zvb0
+  TI *r = nullptr, *rr = nullptr;                  // ru / rv, ruu / rvv
+  double kappa = 0.0, avmmol = 0.0, min_depth = 0.0;
+  int runtype = 0;
+  __host__ __device__ int mask_at(long long c) const { return sizeof(TI) == 4 ? (int)mask8[c] : mask32[c]; }
+  __host__ __device__ int au_at(long long c) const { return sizeof(TI) == 4 ? (int)au8[c] : au32[c]; }
 };
-// both components in one launch (mu / mv: the U and the V grid's flux-u, flux-v, update-u,
-// update-v masks; bfu / bfv: their bottom friction, may be null)
-int run_uvadv2d_both_f32(const Dev& d, cudaStream_t s, float dt, int scheme, const float* U, const float* V,
-                         const float* DU, const float* DV, const uint8_t* const* mu, const uint8_t* const* mv,
-                         float* UEx, float* VEx, const Bf2Args* bfu, const Bf2Args* bfv);
-// bf (may be null): also form the bottom friction of the micro step for this component's points
-int run_uvadv2d_fused_f32(const Dev& d, cudaStream_t s, int dir, float dt, int scheme, const float* U,
-                          const float* V, const float* DU, const float* DV, const uint8_t* mflux_u,
-                          const uint8_t* mflux_v, const uint8_t* mupd_u, const uint8_t* mupd_v, float* Ex,
-                          const Bf2Args* bf = nullptr);
+// mu / mv: the U and the V grid's flux-u, flux-v, update-u, update-v masks
+template <class T, class TI>
+int run_uvadv2d(const Dev& d, cudaStream_t s, T dt, int scheme, const TI* U, const TI* V, const TI* DU, const TI* DV,
+                const uint8_t* const* mu, const uint8_t* const* mv, TI* UEx, TI* VEx, const Bf2Args<TI>* bfu,
+                const Bf2Args<TI>* bfv);
 
 // Vertical sweep of two tracers in place (H_TAG, no sub-iterations), heights updated once.
 template <class R>
