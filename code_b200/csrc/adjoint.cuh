@@ -60,6 +60,7 @@ __global__ void k_adj_heights(Dev d, R dt, int sub, int has_w, const R* __restri
                               const R* __restrict__ vv, const R* __restrict__ ww,
                               const uint8_t* __restrict__ mupd_u, const uint8_t* __restrict__ mupd_v,
                               const int32_t* __restrict__ az, R* H1, R* H2, R* H3, R* H4) {
+  chain_sync();
   const int ii = blockIdx.x * blockDim.x + threadIdx.x;
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = 1 + blockIdx.z;
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(TU) k_adj_sweep_u(Dev d, R dt, R splitfac, R A
                                                     const R* __restrict__ DU, const uint8_t* __restrict__ mflux,
                                                     const uint8_t* __restrict__ mupd,
                                                     const uint8_t* __restrict__ code) {
+  chain_sync();
   __shared__ R sU[2][TU + 5], sDU[2][TU + 5];
   __shared__ R sG[2][TU + 4], sD[2][TU + 4];
   __shared__ uint8_t scd[2][TU + 3];
@@ -221,6 +223,7 @@ __global__ void __launch_bounds__(TVX * TVY) k_adj_sweep_v(Dev d, R dt, R splitf
                                                            const uint8_t* __restrict__ mflux,
                                                            const uint8_t* __restrict__ mupd,
                                                            const uint8_t* __restrict__ code) {
+  chain_sync();
   __shared__ R sV[2][TVY + 5][TVX], sDV[2][TVY + 5][TVX];
   __shared__ R sG[2][TVY + 4][TVX], sD[2][TVY + 4][TVX];
   __shared__ uint8_t scd[2][TVY + 3][TVX];
@@ -351,6 +354,7 @@ __global__ void __launch_bounds__(32 * UWB) k_adj_sweep_u_vec(Dev d, R dt, R spl
                                                             const uint8_t* __restrict__ mflux,
                                                             const uint8_t* __restrict__ mupd,
                                                             const uint8_t* __restrict__ code) {
+  chain_sync();
   static_assert(sizeof(R) == 4, "vectorised adjoint sweeps are FP32");
   constexpr int N = 4;
   constexpr int NA = 5;  // gbar, Dio, U, DU, codes
@@ -499,6 +503,7 @@ __global__ void __launch_bounds__(32 * VKW) k_adj_sweep_v_vec(Dev d, R dt, R spl
                                                             const uint8_t* __restrict__ mflux,
                                                             const uint8_t* __restrict__ mupd,
                                                             const uint8_t* __restrict__ code) {
+  chain_sync();
   static_assert(sizeof(R) == 4, "vectorised adjoint sweeps are FP32");
   constexpr int N = VN;  // cells per lane (4: float4; 2: float2, half the registers)
   constexpr int VB = N * (int)sizeof(R);
@@ -707,6 +712,7 @@ __global__ void __launch_bounds__(128) k_adj_sweep_w(Dev d, R dt, R splitfac, in
                                                      R* __restrict__ fbar, const R* __restrict__ hi,
                                                      const R* __restrict__ ww, const int32_t* __restrict__ az,
                                                      const uint8_t* __restrict__ code) {
+  chain_sync();
   const int ii = blockIdx.x * blockDim.x + threadIdx.x;
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
   if (ii >= d.ni() || jj >= d.nj()) return;
@@ -785,6 +791,7 @@ __global__ void __launch_bounds__(128) k_adj_vdiff(Dev d, R dt, R cnpar, R avmol
                                                    const R* __restrict__ Sn, const R* __restrict__ hn,
                                                    const R* __restrict__ nuh, const int32_t* __restrict__ az,
                                                    R* RUs, R* QUs) {
+  chain_sync();
   const int ii = blockIdx.x * blockDim.x + threadIdx.x;
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
   if (ii >= d.ni() || jj >= d.nj()) return;
@@ -890,8 +897,8 @@ int run_adj_heights(const Dev& d, cudaStream_t s, R dt, int sub, bool has_w, con
   if (d.kmax < 1) return 0;
   dim3 blk(64, 4, 1);
   dim3 grd((d.ni() + blk.x - 1) / blk.x, (d.nj() + blk.y - 1) / blk.y, d.kmax);
-  k_adj_heights<R><<<grd, blk, 0, s>>>(d, dt, sub, has_w ? 1 : 0, ho, uu, vv, ww, mupd_u, mupd_v, az, H1, H2,
-                                       H3, H4);
+  launch_chained(k_adj_heights<R>, grd, blk, 0, s, d, dt, sub, has_w ? 1 : 0, ho, uu, vv, ww, mupd_u, mupd_v, az, H1,
+                 H2, H3, H4);
   return (int)cudaGetLastError();
 }
 
@@ -909,8 +916,8 @@ int run_adj_sweep_h(const Dev& d, cudaStream_t s, int nk, R dt, R splitfac, int 
         const int nseg = (d.ni() + UOWN * N - 1) / (UOWN * N);
         dim3 blk(32, UWB, 1);
         dim3 grd((nseg + UWB - 1) / UWB, d.nj(), nz);
-        k_adj_sweep_u_vec<R, S><<<grd, blk, 0, s>>>(d, dt, splitfac, AH, nk, copy0, gbar, fbar, Dio, U, DU, mflux,
-                                                    mupd, code);
+        launch_chained(k_adj_sweep_u_vec<R, S>, grd, blk, 0, s, d, dt, splitfac, AH, nk, copy0, gbar, fbar, Dio, U,
+                       DU, mflux, mupd, code);
         return (int)cudaGetLastError();
       }
       if (DIR == 1 && vec_layout<R>(d, nk + (copy0 ? 1 : 0), {gbar, fbar, Dio, U, DU}, {mflux, mupd, code})) {
@@ -920,20 +927,20 @@ int run_adj_sweep_h(const Dev& d, cudaStream_t s, int nk, R dt, R splitfac, int 
         while (rows > 8 && nx * ((d.nj() + rows - 1) / rows) * nzv * VKW < 148LL * 24) rows /= 2;
         dim3 blk(32, VKW, 1);
         dim3 grd((unsigned)nx, (d.nj() + rows - 1) / rows, (unsigned)nzv);
-        k_adj_sweep_v_vec<R, S, 2><<<grd, blk, 0, s>>>(d, dt, splitfac, AH, nk, rows, copy0, gbar, fbar, Dio, U, DU,
-                                                    mflux, mupd, code);
+        launch_chained(k_adj_sweep_v_vec<R, S, 2>, grd, blk, 0, s, d, dt, splitfac, AH, nk, rows, copy0, gbar, fbar,
+                       Dio, U, DU, mflux, mupd, code);
         return (int)cudaGetLastError();
       }
     }
     if (DIR == 0) {
       dim3 grd((d.ni() + TU - 1) / TU, d.nj(), nz);
-      k_adj_sweep_u<R, S><<<grd, TU, 0, s>>>(d, dt, splitfac, AH, nk, copy0, gbar, fbar, Dio, U, DU, mflux, mupd,
-                                             code);
+      launch_chained(k_adj_sweep_u<R, S>, grd, TU, 0, s, d, dt, splitfac, AH, nk, copy0, gbar, fbar, Dio, U, DU,
+                     mflux, mupd, code);
     } else {
       dim3 blk(TVX, TVY, 1);
       dim3 grd((d.ni() + TVX - 1) / TVX, (d.nj() + TVY - 1) / TVY, nz);
-      k_adj_sweep_v<R, S><<<grd, blk, 0, s>>>(d, dt, splitfac, AH, nk, copy0, gbar, fbar, Dio, U, DU, mflux, mupd,
-                                              code);
+      launch_chained(k_adj_sweep_v<R, S>, grd, blk, 0, s, d, dt, splitfac, AH, nk, copy0, gbar, fbar, Dio, U, DU,
+                     mflux, mupd, code);
     }
     return (int)cudaGetLastError();
   });
@@ -946,7 +953,7 @@ int run_adj_sweep_w(const Dev& d, cudaStream_t s, R dt, R splitfac, int scheme, 
     constexpr int S = decltype(sc)::value;
     dim3 blk(64, 2, 1);
     dim3 grd((d.ni() + blk.x - 1) / blk.x, (d.nj() + blk.y - 1) / blk.y, 1);
-    k_adj_sweep_w<R, S><<<grd, blk, 0, s>>>(d, dt, splitfac, kshift, gbar, fbar, hi, ww, az, code);
+    launch_chained(k_adj_sweep_w<R, S>, grd, blk, 0, s, d, dt, splitfac, kshift, gbar, fbar, hi, ww, az, code);
     return (int)cudaGetLastError();
   });
 }
@@ -956,7 +963,7 @@ int run_adj_vdiff(const Dev& d, cudaStream_t s, R dt, R cnpar, R avmol, const R*
                   const R* g, const R* Sn, const R* hn, const R* nuh, const int32_t* az, R* rus, R* qus) {
   dim3 blk(32, 4, 1);
   dim3 grd((d.ni() + blk.x - 1) / blk.x, (d.nj() + blk.y - 1) / blk.y, 1);
-  k_adj_vdiff<R><<<grd, blk, 0, s>>>(d, dt, cnpar, avmol, fbar, gbar, nubar, g, Sn, hn, nuh, az, rus, qus);
+  launch_chained(k_adj_vdiff<R>, grd, blk, 0, s, d, dt, cnpar, avmol, fbar, gbar, nubar, g, Sn, hn, nuh, az, rus, qus);
   return (int)cudaGetLastError();
 }
 

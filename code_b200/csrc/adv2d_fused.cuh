@@ -310,6 +310,7 @@ __global__ void __launch_bounds__(TL::FT, (sizeof(TI) == 4 ? 2048 : 1024) / TL::
     k_uvadv2d_both(Dev d, T dt, const TI* __restrict__ U, const TI* __restrict__ V, const TI* __restrict__ DU,
                    const TI* __restrict__ DV, Adv2dMasks mu, Adv2dMasks mv, TI* __restrict__ UEx, TI* __restrict__ VEx,
                    Bf2Args<TI> bfu, Bf2Args<TI> bfv) {
+  chain_sync();
   if (blockIdx.z == 0)
     uvadv2d_tile<TL, T, S, 0, TI>(d, dt, U, V, DU, DV, mu.mflux_u, mu.mflux_v, mu.mupd_u, mu.mupd_v, UEx, bfu);
   else
@@ -332,10 +333,9 @@ int run_uvadv2d(const Dev& d, cudaStream_t s, T dt, int scheme, const TI* U, con
         if (e != cudaSuccess) return (int)e;
       }
       const dim3 grd((d.ni() + TL::FX - 1) / TL::FX, (d.nj() + TL::FY - 1) / TL::FY, 2);
-      kern<<<grd, dim3(TL::RW, TL::FTY, 1), smem, s>>>(
-          d, dt, U, V, DU, DV, Adv2dMasks{mu[0], mu[1], mu[2], mu[3]}, Adv2dMasks{mv[0], mv[1], mv[2], mv[3]}, UEx, VEx,
-          bfu ? *bfu : Bf2Args<TI>{}, bfv ? *bfv : Bf2Args<TI>{});
-      return (int)cudaGetLastError();
+      return launch_chained(kern, grd, dim3(TL::RW, TL::FTY, 1), smem, s, d, dt, U, V, DU, DV,
+                            Adv2dMasks{mu[0], mu[1], mu[2], mu[3]}, Adv2dMasks{mv[0], mv[1], mv[2], mv[3]}, UEx, VEx,
+                            bfu ? *bfu : Bf2Args<TI>{}, bfv ? *bfv : Bf2Args<TI>{});
     };
     const long long large = 2LL * ((d.ni() + TileLarge::FX - 1) / TileLarge::FX) *
                             ((d.nj() + TileLarge::FY - 1) / TileLarge::FY);

@@ -346,6 +346,7 @@ __device__ __forceinline__ void right_of(const R (&v)[N], R (&r)[N]) {
 
 template <class R, int S, bool REC, int NF, int N, bool LO, int MOM>
 __global__ void __launch_bounds__(32 * AW, adv_blocks<R>()) k_adv_uv(Dev d, AdvC<R> C, AdvF<R, NF> F, int rows) {
+  chain_sync();
   constexpr int VB = N * (int)sizeof(R);
   constexpr int LH = LaneSplit<N>::LH, OWN = 32 - LH - LaneSplit<N>::rh_uv;
   constexpr int sub = (S == UPSTREAM) ? 0 : 1;
@@ -547,6 +548,7 @@ __global__ void __launch_bounds__(32 * AW, adv_blocks<R>()) k_adv_uv(Dev d, AdvC
 
 template <class R, int S, bool REC, int NF, int N, bool LO, int MOM>
 __global__ void __launch_bounds__(32 * AW, adv_blocks<R>()) k_adv_vu(Dev d, AdvC<R> C, AdvF<R, NF> F, int rows) {
+  chain_sync();
   constexpr int VB = N * (int)sizeof(R);
   constexpr int LH = LaneSplit<N>::LH, OWN = 32 - LH - LaneSplit<N>::template rh_vu<MOM>();
   constexpr int sub = (S == UPSTREAM) ? 0 : 1;

@@ -56,6 +56,7 @@ __device__ __forceinline__ bool interior(const Dev& d, int i, int j) {
 // (inputs and outputs stay FP64 arrays).
 template <class T, bool MIX>
 __global__ void k_bottom_friction(Dev d, Bc2 s, Bc2W w, int runtype) {
+  chain_sync();
   GB_IJ2
   auto U = f2a<MIX, U_>(d, s, w);
   auto V = f2a<MIX, V_>(d, s, w);
@@ -124,6 +125,7 @@ __global__ void k_bottom_friction(Dev d, Bc2 s, Bc2W w, int runtype) {
 // MIX: the roughness arrays are the FP32 working copies.
 template <bool MIX>
 __global__ void __launch_bounds__(256) k_bottom_friction_f32t(Dev d, Bc2 s, Bc2W w, int runtype) {
+  chain_sync();
   __shared__ float suq[10][34], svq[10][34];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i0 = blockIdx.x * 32 + d.imin - HALO, j0 = blockIdx.y * 8 + d.jmin - HALO;
@@ -187,6 +189,7 @@ __global__ void __launch_bounds__(256) k_bottom_friction_f32t(Dev d, Bc2 s, Bc2W
 template <int DIR, class T>
 __global__ void k_uvadv2d_prep(Dev d, const double* Up, const double* Vp, const double* DUp, const double* DVp,
                                T* fadv, T* Uadv, T* Vadv, T* DUadv, T* DVadv, T* Do) {
+  chain_sync();
   GB_IJ2
   W2 U{d, const_cast<double*>(Up)}, V{d, const_cast<double*>(Vp)}, DU_{d, const_cast<double*>(DUp)},
       DV_{d, const_cast<double*>(DVp)};
@@ -211,6 +214,7 @@ __global__ void k_uvadv2d_prep(Dev d, const double* Up, const double* Vp, const 
 
 // FP32 advective increments of the mixed step widened into the FP64 UEx / VEx
 __global__ void k_widen2d(Dev d, const float* a, double* out) {
+  chain_sync();
   GB_IJ2
   const long long c = d.ix(i, j);
   out[c] = (double)a[c];
@@ -219,6 +223,7 @@ __global__ void k_widen2d(Dev d, const float* a, double* out) {
 // NOSPLIT finaliser of the 2D driver (advection.F90:500-507)
 template <class T>
 __global__ void k_finalise2d(Dev d, T dt, T* f, const T* Do, const T* adv, const T* Di, const uint8_t* mfin) {
+  chain_sync();
   GB_IJ2
   const long long c = d.ix(i, j);
   if (mfin[c]) f[c] = (Do[c] * f[c] - dt * adv[c]) / Di[c];
@@ -233,6 +238,7 @@ __global__ void k_finalise2d(Dev d, T dt, T* f, const T* Do, const T* adv, const
 // point reads a value another thread changes).
 template <int DIR, bool MIX, bool COR = false>
 __global__ void k_momentum(Dev d, Bc2 s, Bc2W w) {
+  chain_sync();
   GB_IJ2
   if (!interior(d, i, j)) return;
   if constexpr (COR) {
@@ -345,6 +351,7 @@ __device__ __forceinline__ float momentum_new_f32(const Dev& d, const Bc2& s, co
 
 template <int DIR, bool COR>
 __global__ void k_momentum_f32(Dev d, Bc2 s, Bc2W w) {
+  chain_sync();
   GB_IJ2
   if (!interior(d, i, j)) return;
   const long long c = d.ix(i, j);
@@ -371,6 +378,7 @@ __device__ __forceinline__ float2 ld_f2(const float* p) { return *reinterpret_ca
 __device__ __forceinline__ double2 ld_d2(const double* p) { return *reinterpret_cast<const double2*>(p); }
 template <int DIR, bool COR>
 __global__ void k_momentum_f32v(Dev d, Bc2 s, Bc2W w) {
+  chain_sync();
   const int ii = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
   if (ii >= d.ni() || jj >= d.nj()) return;
@@ -459,6 +467,7 @@ __global__ void k_momentum_f32v(Dev d, Bc2 s, Bc2W w) {
 // momentum.F90:193-216 / :356-379: Coriolis terms fU (after the U update) and fV (after V).
 template <int DIR, bool MIX>
 __global__ void k_coriolis(Dev d, Bc2 s, Bc2W w) {
+  chain_sync();
   GB_IJ2
   if (!interior(d, i, j)) return;
   if constexpr (MIX) {  // FP32 arithmetic on the working copies, as k_momentum_f32 forms the terms
@@ -502,6 +511,7 @@ __global__ void k_coriolis(Dev d, Bc2 s, Bc2W w) {
 // m2d.F90:471-472 (Uint, Vint accumulation, FP64) + sealevel.F90:89-112 (zo = z; z update).
 template <bool MIX>
 __global__ void k_accum_sealevel(Dev d, Bc2 s, Bc2W w, int accumulate) {
+  chain_sync();
   GB_IJ2
   auto U = f2a<MIX, U_>(d, s, w);
   auto V = f2a<MIX, V_>(d, s, w);
@@ -524,6 +534,7 @@ __global__ void k_accum_sealevel(Dev d, Bc2 s, Bc2W w, int accumulate) {
 // depth_update.F90:55-110
 template <bool MIX>
 __global__ void k_depth_update(Dev d, Bc2 s, Bc2W w) {
+  chain_sync();
   GB_IJ2
   auto D = f2a<MIX, D_>(d, s, w);
   auto DU_ = f2a<MIX, DU>(d, s, w);
@@ -565,6 +576,7 @@ __global__ void k_depth_update(Dev d, Bc2 s, Bc2W w) {
 // for it on the micro steps whose state a macro step or the host reads next.
 template <bool MIX>
 __global__ void k_sealevel_depth(Dev d, Bc2 s, Bc2W w, int flags) {
+  chain_sync();
   const int accumulate = flags & 1;
   GB_IJ2
   auto U = f2a<MIX, U_>(d, s, w);
@@ -622,6 +634,7 @@ __global__ void k_sealevel_depth(Dev d, Bc2 s, Bc2W w, int flags) {
 // formed once each (the one-point form forms three per point). The same expressions, so the same
 // values; every load stays inside the haloed plane (the conditions are those of the one-point form).
 __global__ void k_sealevel_depth_p(Dev d, Bc2 s, Bc2W w, int flags) {
+  chain_sync();
   const int ii = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
   if (ii >= d.ni() || jj >= d.nj()) return;
@@ -730,6 +743,7 @@ __global__ void k_sealevel_depth_p(Dev d, Bc2 s, Bc2W w, int flags) {
 
 // exchanges the contents of two 2D FP64 arrays (the elevation ping-pong's last state)
 __global__ void k_swap2(long long n2, double* a, double* b) {
+  chain_sync();
   for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n2; c += (long long)gridDim.x * blockDim.x) {
     const double x = a[c];
     a[c] = b[c];
@@ -739,6 +753,7 @@ __global__ void k_swap2(long long n2, double* a, double* b) {
 
 // start_macro.F90:54-86, first loop (T points) ...
 __global__ void k_start_macro_t(Dev d, Bc2 s) {
+  chain_sync();
   GB_IJ2
   W2 sseo{d, s.f2[SSEO]}, ssen{d, s.f2[SSEN]}, z{d, s.f2[Z]}, Dn{d, s.f2[DN]}, H{d, s.f2[HH]};
   sseo(i, j) = ssen(i, j);
@@ -747,6 +762,7 @@ __global__ void k_start_macro_t(Dev d, Bc2 s) {
 }
 // ... then U and V points and Uint/M, Vint/M
 __global__ void k_start_macro_uv(Dev d, Bc2 s, double split) {
+  chain_sync();
   GB_IJ2
   W2 sseo{d, s.f2[SSEO]}, ssen{d, s.f2[SSEN]}, ssuo{d, s.f2[SSUO]}, ssun{d, s.f2[SSUN]}, HU_{d, s.f2[HU]},
       Dun{d, s.f2[DUN]}, ssvo{d, s.f2[SSVO]}, ssvn{d, s.f2[SSVN]}, HV_{d, s.f2[HV]}, Dvn{d, s.f2[DVN]},
@@ -772,6 +788,7 @@ __global__ void k_start_macro_uv(Dev d, Bc2 s, double split) {
 
 // slow_bottom_friction.F90:53-93: depth-averaged velocities of the last macro step (scratch Ui/Vi)
 __global__ void k_sbf_uv(Dev d, Bc2 s, double* Uip, double* Vip) {
+  chain_sync();
   GB_IJ2
   W2 Uinto{d, s.f2[UINTO]}, Vinto{d, s.f2[VINTO]}, ssuo{d, s.f2[SSUO]}, ssvo{d, s.f2[SSVO]}, HU_{d, s.f2[HU]},
       HV_{d, s.f2[HV]}, Ui{d, Uip}, Vi{d, Vip};
@@ -790,6 +807,7 @@ __global__ void k_sbf_uv(Dev d, Bc2 s, double* Uip, double* Vip) {
 // slow_bottom_friction.F90:95-170: ru, rv of the slow (macro) friction. Counts non-positive log
 // arguments (the reference stops with 'Bottom friction coefficient infinite').
 __global__ void k_sbf_r(Dev d, Bc2 s, const double* Uip, const double* Vip, unsigned long long* bad) {
+  chain_sync();
   GB_IJ2
   if (!interior(d, i, j)) return;
   W2 ssun{d, s.f2[SSUN]}, ssvn{d, s.f2[SSVN]}, HU_{d, s.f2[HU]}, HV_{d, s.f2[HV]}, zub{d, s.f2[ZUB]},
@@ -828,6 +846,7 @@ __global__ void k_sbf_r(Dev d, Bc2 s, const double* Uip, const double* Vip, unsi
 __global__ void k_bdy2d(Dev d, Bc2 s, const int4* __restrict__ pts, int p0, int p1, const double* data,
                         const double* data_u, const double* data_v, const double* amp, const double* phase,
                         double period, double fac, int loop) {
+  chain_sync();
   const int p = p0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= p1) return;
   W2 z{d, s.f2[Z]}, D{d, s.f2[D_]}, U{d, s.f2[U_]}, DU_{d, s.f2[DU]}, V{d, s.f2[V_]}, DV_{d, s.f2[DV]},
@@ -890,6 +909,7 @@ __global__ void k_bdy2d(Dev d, Bc2 s, const int4* __restrict__ pts, int p0, int 
 // on nl levels with stride sk.
 template <class T>
 __global__ void k_mirror(T* f, const long long* __restrict__ pairs, int n, int nl, long long sk) {
+  chain_sync();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n) return;
   const long long dst = pairs[2 * p], src = pairs[2 * p + 1];
@@ -902,6 +922,7 @@ __global__ void k_mirror(T* f, const long long* __restrict__ pairs, int n, int n
 // With `latched`, cnt[2] != 0 (a finding of an earlier sweep: the reference's have_warned) skips the
 // sweep.
 __global__ void k_nan_sweep(Dev d, const double* __restrict__ z, unsigned long long* cnt, bool latched) {
+  chain_sync();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + d.imin;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + d.jmin;
   if (i > d.imax || j > d.jmax) return;
@@ -920,6 +941,7 @@ __global__ void k_nan_sweep(Dev d, const double* __restrict__ z, unsigned long l
 // (cppdefs.h:161-170, _2D_W_HOT_ / _3D_W_HOT_).
 template <class R>
 __global__ void k_interior_copy(Dev d, R* f, double* buf, int nl, int to_buf) {
+  chain_sync();
   const int nx = d.imax - d.imin + 1, ny = d.jmax - d.jmin + 1;
   const long long n = (long long)nx * ny * nl;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -935,6 +957,7 @@ __global__ void k_interior_copy(Dev d, R* f, double* buf, int nl, int to_buf) {
 // postinit_2d (m2d.F90:358-390), first half: flag[0] = 1 if any U /= 0 where au == 0 or V /= 0 where
 // av == 0 (haloed plane)
 __global__ void k_hot_check(Dev d, Bc2 s, unsigned long long* flag) {
+  chain_sync();
   GB_IJ2
   M2 au{d, s.au}, av{d, s.av};
   W2 U{d, s.f2[U_]}, V{d, s.f2[V_]};
@@ -944,6 +967,7 @@ __global__ void k_hot_check(Dev d, Bc2 s, unsigned long long* flag) {
 // postinit_2d (m2d.F90:380-396): the reset of U, Uinto / V, Vinto on closed velocity points when the
 // check found any, and the elevations of land points set to -9999
 __global__ void k_hot_reset2d(Dev d, Bc2 s, const unsigned long long* flag) {
+  chain_sync();
   GB_IJ2
   M2 az{d, s.az}, au{d, s.au}, av{d, s.av};
   W2 U{d, s.f2[U_]}, V{d, s.f2[V_]}, Uinto{d, s.f2[UINTO]}, Vinto{d, s.f2[VINTO]}, z{d, s.f2[Z]}, zo{d, s.f2[ZO]};
@@ -967,6 +991,7 @@ __global__ void k_hot_reset2d(Dev d, Bc2 s, const unsigned long long* flag) {
 // tke = 0, num = nuh = 1e-15 (single-precision literal), T = S = -9999; every level
 template <class R3>
 __global__ void k_hot_reset3d(Dev d, Bc2 s, R3* uu, R3* vv, R3* tke, R3* num, R3* nuh, R3* T, R3* S) {
+  chain_sync();
   GB_IJ2
   M2 az{d, s.az}, au{d, s.au}, av{d, s.av};
   const long long c = d.ix(i, j);
@@ -986,6 +1011,7 @@ __global__ void k_hot_reset3d(Dev d, Bc2 s, R3* uu, R3* vv, R3* tke, R3* num, R3
 
 // stop_macro.F90:36-39
 __global__ void k_stop_macro(Dev d, Bc2 s) {
+  chain_sync();
   GB_IJ2
   W2 Uint{d, s.f2[UINT]}, Vint{d, s.f2[VINT]}, Uinto{d, s.f2[UINTO]}, Vinto{d, s.f2[VINTO]};
   Uinto(i, j) = Uint(i, j);
@@ -1000,6 +1026,7 @@ namespace gb {
 
 // after a sweep: a finding ends the sweeps (the reference's have_warned)
 __global__ void k_nan_latch(unsigned long long* cnt) {
+  chain_sync();
   if (cnt[0] != 0) cnt[2] = 1;
 }
 
@@ -1007,15 +1034,15 @@ __global__ void k_nan_latch(unsigned long long* cnt) {
 int run_nan_sweep_once(const Dev& d, cudaStream_t s, const double* z, unsigned long long* cnt) {
   const dim3 blk(32, 4, 1);
   const dim3 g((d.imax - d.imin + 1 + 31) / 32, (d.jmax - d.jmin + 1 + 3) / 4, 1);
-  k_nan_sweep<<<g, blk, 0, s>>>(d, z, cnt, false);
+  launch_chained(k_nan_sweep, g, blk, 0, s, d, z, cnt, false);
   return (int)cudaGetLastError();
 }
 
 int run_nan_sweep(const Dev& d, cudaStream_t s, const double* z, unsigned long long* cnt) {
   const dim3 blk(32, 4, 1);
   const dim3 g((d.imax - d.imin + 1 + 31) / 32, (d.jmax - d.jmin + 1 + 3) / 4, 1);
-  k_nan_sweep<<<g, blk, 0, s>>>(d, z, cnt, true);
-  k_nan_latch<<<1, 1, 0, s>>>(cnt);
+  launch_chained(k_nan_sweep, g, blk, 0, s, d, z, cnt, true);
+  launch_chained(k_nan_latch, 1, 1, 0, s, cnt);
   return (int)cudaGetLastError();
 }
 
@@ -1087,9 +1114,9 @@ int mirror_bdy(getm_ctx* ctx, T* f, int tag, int nl) {
     const int p0 = b.pair_first[tag][side], p1 = b.pair_first[tag][side + 1];
     if (p1 <= p0) continue;
     TimerScope ts(ctx, nl > 1 ? GETM_TIM_BC3D : GETM_TIM_BC2D);
-    k_mirror<T><<<(p1 - p0 + 127) / 128, 128, 0, ctx->stream>>>(f, b.pairs + 2 * (long long)p0, p1 - p0, nl,
-                                                                ctx->dev.sk);
-    GB_TRY(cudaGetLastError(), "mirror_bdy");
+    GB_TRY(launch_chained(k_mirror<T>, (p1 - p0 + 127) / 128, 128, 0, ctx->stream, f, b.pairs + 2 * (long long)p0,
+                          p1 - p0, nl, ctx->dev.sk),
+           "mirror_bdy");
   }
   return GETM_OK;
 }
@@ -1104,10 +1131,9 @@ int bdy_2d(getm_ctx* ctx, const Bc2& s, int loop) {
     const int p0 = b.side_first[side], p1 = b.side_first[side + 1];
     if (p1 <= p0) continue;
     TimerScope ts(ctx, GETM_TIM_BC2D);
-    k_bdy2d<<<(p1 - p0 + 127) / 128, 128, 0, ctx->stream>>>(ctx->dev, s, b.pts, p0, p1, b.data, b.data_u, b.data_v,
-                                                            b.harmonic ? b.amp : nullptr, b.phase, b.period, fac,
-                                                            loop);
-    GB_TRY(cudaGetLastError(), "update_2d_bdy");
+    GB_TRY(launch_chained(k_bdy2d, (p1 - p0 + 127) / 128, 128, 0, ctx->stream, ctx->dev, s, b.pts, p0, p1, b.data,
+                          b.data_u, b.data_v, b.harmonic ? b.amp : nullptr, b.phase, b.period, fac, loop),
+           "update_2d_bdy");
   }
   return GETM_OK;
 }
@@ -1166,7 +1192,7 @@ int do_adv2d(getm_ctx* ctx, T dt, T* f, const T* U, const T* V, const T* DUa, co
       GB_TIMED(GETM_TIM_BC2D, (run_sweep_h<T, 1>(d, s, 1, dt, one, scheme, zero, f, S, S, Di, Di, A, V, DVa,
                                                   g.mask_vflux, g.mask_vupdate)), "v");
       if (need_f) {
-        k_finalise2d<T><<<grid2(d), kBlk2, 0, s>>>(d, dt, f, Do, A, Di, g.mask_finalise);
+        launch_chained(k_finalise2d<T>, grid2(d), kBlk2, 0, s, d, dt, f, Do, A, Di, g.mask_finalise);
         GB_TRY(cudaGetLastError(), "finalise2d");
       }
       break;
@@ -1269,11 +1295,11 @@ int uv_advect_2d_t(getm_ctx* ctx, const getm_bc_state* st, const double* U, cons
     {
       TimerScope ts(ctx, GETM_TIM_BC2D);
       if (dir == 0)
-        k_uvadv2d_prep<0, T><<<grid2(d), kBlk2, 0, s>>>(d, U, V, DU_, DV_, fadv, Uadv, Vadv, DUadv, DVadv,
-                                                         is64 ? nullptr : Do);
+        launch_chained(k_uvadv2d_prep<0, T>, grid2(d), kBlk2, 0, s, d, U, V, DU_, DV_, fadv, Uadv, Vadv, DUadv, DVadv,
+                       is64 ? nullptr : Do);
       else
-        k_uvadv2d_prep<1, T><<<grid2(d), kBlk2, 0, s>>>(d, U, V, DU_, DV_, fadv, Uadv, Vadv, DUadv, DVadv,
-                                                         is64 ? nullptr : Do);
+        launch_chained(k_uvadv2d_prep<1, T>, grid2(d), kBlk2, 0, s, d, U, V, DU_, DV_, fadv, Uadv, Vadv, DUadv, DVadv,
+                       is64 ? nullptr : Do);
       GB_TRY(cudaGetLastError(), "uv_advect prep");
     }
     const T* Dsrc = is64 ? (const T*)(dir == 0 ? DU_ : DV_) : Do;
@@ -1282,7 +1308,7 @@ int uv_advect_2d_t(getm_ctx* ctx, const getm_bc_state* st, const double* U, cons
     if (rc) return rc;
     if (!is64) {
       TimerScope ts(ctx, GETM_TIM_BC2D);
-      k_widen2d<<<grid2(d), kBlk2, 0, s>>>(d, (const float*)A, Ex[dir]);
+      launch_chained(k_widen2d, grid2(d), kBlk2, 0, s, d, (const float*)A, Ex[dir]);
       GB_TRY(cudaGetLastError(), "widen");
     }
   }
@@ -1298,7 +1324,7 @@ int uv_advect_2d(getm_ctx* ctx, const getm_bc_state* st, const double* U, const 
 #define GB_K2(kernel, ...)                                         \
   do {                                                             \
     TimerScope _ts(ctx, GETM_TIM_BC2D);                            \
-    kernel<<<grid2(d), kBlk2, 0, ctx->stream>>>(__VA_ARGS__);      \
+    launch_chained(kernel, grid2(d), kBlk2, 0, ctx->stream, __VA_ARGS__);      \
     GB_TRY(cudaGetLastError(), #kernel);                           \
   } while (0)
 
@@ -1343,9 +1369,10 @@ int bottom_friction_2d(getm_ctx* ctx, const getm_bc_state* st, int runtype, cons
   const Bc2W w = wp ? *wp : Bc2W{};
   const dim3 gt((d.ni() + 31) / 32, (d.nj() + 7) / 8, 1);
   TimerScope ts(ctx, GETM_TIM_BC2D);
-  if (wp) k_bottom_friction_f32t<true><<<gt, dim3(32, 8, 1), 0, ctx->stream>>>(d, s, w, runtype);
-  else if (st->prec3d == 8) k_bottom_friction<double, false><<<grid2(d), kBlk2, 0, ctx->stream>>>(d, s, w, runtype);
-  else k_bottom_friction_f32t<false><<<gt, dim3(32, 8, 1), 0, ctx->stream>>>(d, s, w, runtype);
+  if (wp) launch_chained(k_bottom_friction_f32t<true>, gt, dim3(32, 8, 1), 0, ctx->stream, d, s, w, runtype);
+  else if (st->prec3d == 8) launch_chained(k_bottom_friction<double, false>, grid2(d), kBlk2, 0, ctx->stream, d, s, w,
+                                           runtype);
+  else launch_chained(k_bottom_friction_f32t<false>, gt, dim3(32, 8, 1), 0, ctx->stream, d, s, w, runtype);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? GETM_OK : cuda_fail(ctx, (int)e, "bottom_friction");
 }
@@ -1379,23 +1406,23 @@ int momentum_2d(getm_ctx* ctx, const getm_bc_state* st, const Bc2W* wp, bool cor
   cudaStream_t cs = ctx->stream;
   {
     TimerScope ts(ctx, GETM_TIM_BC2D);
-    if (!wp && fused && cor) k_momentum<DIR, false, true><<<grid2(d), kBlk2, 0, cs>>>(d, s, w);
-    else if (!wp) k_momentum<DIR, false><<<grid2(d), kBlk2, 0, cs>>>(d, s, w);
+    int e;
+    if (!wp && fused && cor) e = launch_chained(k_momentum<DIR, false, true>, grid2(d), kBlk2, 0, cs, d, s, w);
+    else if (!wp) e = launch_chained(k_momentum<DIR, false, false>, grid2(d), kBlk2, 0, cs, d, s, w);
     else if (pairs_ok(d, s, w)) {
       const dim3 gp((d.ni() / 2 + 31) / 32, (d.nj() + 3) / 4, 1);
-      if (cor) k_momentum_f32v<DIR, true><<<gp, kBlk2, 0, cs>>>(d, s, w);
-      else k_momentum_f32v<DIR, false><<<gp, kBlk2, 0, cs>>>(d, s, w);
-    } else if (cor) k_momentum_f32<DIR, true><<<grid2(d), kBlk2, 0, cs>>>(d, s, w);
-    else k_momentum_f32<DIR, false><<<grid2(d), kBlk2, 0, cs>>>(d, s, w);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(ctx, (int)e, DIR == 0 ? "umomentum" : "vmomentum");
+      if (cor) e = launch_chained(k_momentum_f32v<DIR, true>, gp, kBlk2, 0, cs, d, s, w);
+      else e = launch_chained(k_momentum_f32v<DIR, false>, gp, kBlk2, 0, cs, d, s, w);
+    } else if (cor) e = launch_chained(k_momentum_f32<DIR, true>, grid2(d), kBlk2, 0, cs, d, s, w);
+    else e = launch_chained(k_momentum_f32<DIR, false>, grid2(d), kBlk2, 0, cs, d, s, w);
+    if (e) return cuda_fail(ctx, e, DIR == 0 ? "umomentum" : "vmomentum");
   }
   if (wp) return GETM_OK;
   int r;
   if ((r = mirror_bdy<double>(ctx, st->f2[DIR == 0 ? U_ : V_], DIR, 1))) return r;
   if (fused) return GETM_OK;
   TimerScope ts(ctx, GETM_TIM_BC2D);
-  k_coriolis<DIR, false><<<grid2(d), kBlk2, 0, cs>>>(d, s, w);
+  launch_chained(k_coriolis<DIR, false>, grid2(d), kBlk2, 0, cs, d, s, w);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? GETM_OK : cuda_fail(ctx, (int)e, "coriolis");
 }
@@ -1415,7 +1442,7 @@ int integrate_2d(getm_ctx* ctx, getm_bc_state* st, int loop, const Bc2W* wp = nu
   const Bc2W w = mix ? *wp : Bc2W{};
   auto k2 = [&](auto kernel, auto... args) -> int {
     TimerScope ts(ctx, GETM_TIM_BC2D);
-    kernel<<<grid2(d), kBlk2, 0, ctx->stream>>>(args...);
+    launch_chained(kernel, grid2(d), kBlk2, 0, ctx->stream, args...);
     return (int)cudaGetLastError();
   };
   int rc = GETM_OK;
@@ -1469,10 +1496,14 @@ int integrate_2d(getm_ctx* ctx, getm_bc_state* st, int loop, const Bc2W* wp = nu
     const int flags = (ip[I_RUNTYPE] > 1 ? 1 : 0) | (dryz ? 2 : 0);
     if (mix && pairs_ok(d, s, w)) {
       TimerScope ts(ctx, GETM_TIM_BC2D);
-      k_sealevel_depth_p<<<dim3((d.ni() / 2 + 31) / 32, (d.nj() + 3) / 4, 1), kBlk2, 0, ctx->stream>>>(d, s, w, flags);
-      rc = (int)cudaGetLastError();
+      rc = launch_chained(k_sealevel_depth_p, dim3((d.ni() / 2 + 31) / 32, (d.nj() + 3) / 4, 1), kBlk2, 0,
+                          ctx->stream, d,
+                          s, w, flags);
     } else {
-      rc = mix ? k2(k_sealevel_depth<true>, d, s, w, flags) : k2(k_sealevel_depth<false>, d, s, w, flags);
+      TimerScope ts(ctx, GETM_TIM_BC2D);
+      rc = launch_chained(mix ? k_sealevel_depth<true> : k_sealevel_depth<false>, grid2(d), kBlk2, 0, ctx->stream, d,
+                          s, w,
+                          flags);
     }
     if (rc) return cuda_fail(ctx, rc, "sealevel + depth_update");
     std::swap(st->f2[Z], st->f2[ZO]);
@@ -1490,6 +1521,7 @@ int integrate_2d(getm_ctx* ctx, getm_bc_state* st, int loop, const Bc2W* wp = nu
 // uint8 copies of the masks az, au, av (values 0..3) for the mixed-precision micro step
 __global__ void k_mask8(long long n2, const int32_t* az, const int32_t* au, const int32_t* av, uint8_t* m8,
                         long long pitch) {
+  chain_sync();
   for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n2; c += (long long)gridDim.x * blockDim.x) {
     m8[c] = (uint8_t)az[c];
     m8[pitch + c] = (uint8_t)au[c];
@@ -1507,6 +1539,7 @@ struct FieldList {
 // The 2D fields are contiguous planes of n2 elements; each grid row (blockIdx.y) copies one field,
 // four elements per thread step (16-byte float4 / two double2 accesses when vec), grid-stride.
 __global__ void k_sync_w2(long long n2, Bc2 s, Bc2W w, FieldList fl, int to_w, int vec) {
+  chain_sync();
   const int q = fl.q[blockIdx.y];
   double* a = s.f2[q];
   float* b = w.w[q];
@@ -1958,7 +1991,7 @@ int getm_sealevel(getm_ctx* ctx, getm_bc_state* st, int loop) {
   const Dev& d = ctx->dev;
   {
     TimerScope ts(ctx, GETM_TIM_BC2D);
-    k_accum_sealevel<false><<<grid2(d), kBlk2, 0, ctx->stream>>>(d, to_bc2(st), Bc2W{}, 0);
+    launch_chained(k_accum_sealevel<false>, grid2(d), kBlk2, 0, ctx->stream, d, to_bc2(st), Bc2W{}, 0);
     GB_TRY(cudaGetLastError(), "sealevel");
   }
   if ((rc = nan_sweep_due(ctx, st, loop))) return rc;
@@ -1969,7 +2002,7 @@ int getm_depth_update(getm_ctx* ctx, getm_bc_state* st) {
   GB_BC_ENTRY;
   const Dev& d = ctx->dev;
   TimerScope ts(ctx, GETM_TIM_BC2D);
-  k_depth_update<false><<<grid2(d), kBlk2, 0, ctx->stream>>>(d, to_bc2(st), Bc2W{});
+  launch_chained(k_depth_update<false>, grid2(d), kBlk2, 0, ctx->stream, d, to_bc2(st), Bc2W{});
   GB_TRY(cudaGetLastError(), "depth_update");
   return GETM_OK;
 }
@@ -2051,8 +2084,9 @@ static int restart_field(getm_ctx* ctx, void* f, int elem, int nl, double* host,
                        "restart upload");
   if (f) {
     TimerScope ts(ctx, GETM_TIM_COPY);
-    if (elem == 8) k_interior_copy<double><<<blocks, 256, 0, ctx->stream>>>(d, (double*)f, ctx->stage, nl, to_host);
-    else k_interior_copy<float><<<blocks, 256, 0, ctx->stream>>>(d, (float*)f, ctx->stage, nl, to_host);
+    if (elem == 8) launch_chained(k_interior_copy<double>, blocks, 256, 0, ctx->stream, d, (double*)f, ctx->stage, nl,
+                                  to_host);
+    else launch_chained(k_interior_copy<float>, blocks, 256, 0, ctx->stream, d, (float*)f, ctx->stage, nl, to_host);
     GB_TRY(cudaGetLastError(), "restart field");
   } else if (to_host) {
     GB_TRY(cudaMemsetAsync(ctx->stage, 0, n * sizeof(double), ctx->stream), "restart field");
@@ -2101,22 +2135,20 @@ int getm_restart_read(getm_ctx* ctx, getm_bc_state* st, int runtype, const doubl
   GB_TRY(cudaMemsetAsync(flag, 0, sizeof(unsigned long long), ctx->stream), "hotstart");
   {
     TimerScope ts(ctx, GETM_TIM_BC2D);
-    k_hot_check<<<grid2(d), kBlk2, 0, ctx->stream>>>(d, s2, flag);
-    k_hot_reset2d<<<grid2(d), kBlk2, 0, ctx->stream>>>(d, s2, flag);
-    k_depth_update<false><<<grid2(d), kBlk2, 0, ctx->stream>>>(d, s2, Bc2W{});
+    launch_chained(k_hot_check, grid2(d), kBlk2, 0, ctx->stream, d, s2, flag);
+    launch_chained(k_hot_reset2d, grid2(d), kBlk2, 0, ctx->stream, d, s2, flag);
+    launch_chained(k_depth_update<false>, grid2(d), kBlk2, 0, ctx->stream, d, s2, Bc2W{});
     GB_TRY(cudaGetLastError(), "postinit_2d");
   }
   if (runtype >= 2) {
     TimerScope ts(ctx, GETM_TIM_BC3D);
     void** f3 = st->f3;
     if (st->prec3d == 8)
-      k_hot_reset3d<double><<<grid2(d), kBlk2, 0, ctx->stream>>>(d, s2, (double*)f3[UU], (double*)f3[VV],
-                                                               (double*)f3[TKE], (double*)f3[NUM], (double*)f3[NUH],
-                                                               (double*)f3[TT], (double*)f3[SS]);
+      launch_chained(k_hot_reset3d<double>, grid2(d), kBlk2, 0, ctx->stream, d, s2, (double*)f3[UU], (double*)f3[VV],
+                     (double*)f3[TKE], (double*)f3[NUM], (double*)f3[NUH], (double*)f3[TT], (double*)f3[SS]);
     else
-      k_hot_reset3d<float><<<grid2(d), kBlk2, 0, ctx->stream>>>(d, s2, (float*)f3[UU], (float*)f3[VV], (float*)f3[TKE],
-                                                              (float*)f3[NUM], (float*)f3[NUH], (float*)f3[TT],
-                                                              (float*)f3[SS]);
+      launch_chained(k_hot_reset3d<float>, grid2(d), kBlk2, 0, ctx->stream, d, s2, (float*)f3[UU], (float*)f3[VV],
+                     (float*)f3[TKE], (float*)f3[NUM], (float*)f3[NUH], (float*)f3[TT], (float*)f3[SS]);
     GB_TRY(cudaGetLastError(), "postinit_3d");
     rc = st->prec3d == 8 ? bc3<double>(ctx, st, BC3_SIGMA, GETM_TIM_BC3D) : bc3<float>(ctx, st, BC3_SIGMA, GETM_TIM_BC3D);
     if (rc) return rc;
@@ -2162,7 +2194,7 @@ int getm_time_loop(getm_ctx* ctx, getm_bc_state* st_user, int n0, int count) {
   if (zswap) {
     std::copy(loc.ipar, loc.ipar + NPI, st_user->ipar);
     if (loc.f2[Z] != st_user->f2[Z]) {
-      k_swap2<<<592, 256, 0, ctx->stream>>>(n2d(ctx->dev), st_user->f2[Z], st_user->f2[ZO]);
+      launch_chained(k_swap2, 592, 256, 0, ctx->stream, n2d(ctx->dev), st_user->f2[Z], st_user->f2[ZO]);
       const cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess && rc == GETM_OK) rc = cuda_fail(ctx, (int)e, "elevation ping-pong");
     }
@@ -2202,7 +2234,7 @@ static int time_loop(getm_ctx* ctx, getm_bc_state* st, int n0, int count, bool z
     }
     uint8_t* m8 = reinterpret_cast<uint8_t*>(ctx->w2) + m8off;
     for (int q = 0; q < 3; ++q) w.m8[q] = m8 + q * m8pitch;
-    k_mask8<<<592, 256, 0, ctx->stream>>>(n2, st->az, st->au, st->av, m8, m8pitch);
+    launch_chained(k_mask8, 592, 256, 0, ctx->stream, n2, st->az, st->au, st->av, m8, m8pitch);
     GB_TRY(cudaGetLastError(), "uint8 masks");
     // written by the micro steps; written by the macro step and read by the micro steps
     for (int q : {U_, V_, D_, DU, DV, DRY_U, DRY_V, FU, FV, RU, RV, RUU, RVV, UEX, VEX}) written |= 1ull << q;
@@ -2220,7 +2252,7 @@ static int time_loop(getm_ctx* ctx, getm_bc_state* st, int n0, int count, bool z
     for (int m = 0; m < fl.n; ++m)
       vec = vec && reinterpret_cast<uintptr_t>(st->f2[fl.q[m]]) % 16 == 0 &&
             reinterpret_cast<uintptr_t>(w.w[fl.q[m]]) % 16 == 0;
-    k_sync_w2<<<dim3(592, fl.n, 1), 256, 0, ctx->stream>>>(n2, to_bc2(st), w, fl, to_w, vec ? 1 : 0);
+    launch_chained(k_sync_w2, dim3(592, fl.n, 1), 256, 0, ctx->stream, n2, to_bc2(st), w, fl, to_w, vec ? 1 : 0);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? GETM_OK : cuda_fail(ctx, (int)e, "mixed-precision 2D copies");
   };
@@ -2248,10 +2280,10 @@ static int time_loop(getm_ctx* ctx, getm_bc_state* st, int n0, int count, bool z
     TimerScope ts(ctx, GETM_TIM_BC2D);
     const Bc2 s2 = to_bc2(st);
     const bool v_last = st->ipar[I_UFIRST2D] == 0;
-    if (mix && v_last) k_coriolis<1, true><<<grid2(ctx->dev), kBlk2, 0, ctx->stream>>>(ctx->dev, s2, w);
-    else if (mix) k_coriolis<0, true><<<grid2(ctx->dev), kBlk2, 0, ctx->stream>>>(ctx->dev, s2, w);
-    else if (v_last) k_coriolis<1, false><<<grid2(ctx->dev), kBlk2, 0, ctx->stream>>>(ctx->dev, s2, w);
-    else k_coriolis<0, false><<<grid2(ctx->dev), kBlk2, 0, ctx->stream>>>(ctx->dev, s2, w);
+    if (mix && v_last) launch_chained(k_coriolis<1, true>, grid2(ctx->dev), kBlk2, 0, ctx->stream, ctx->dev, s2, w);
+    else if (mix) launch_chained(k_coriolis<0, true>, grid2(ctx->dev), kBlk2, 0, ctx->stream, ctx->dev, s2, w);
+    else if (v_last) launch_chained(k_coriolis<1, false>, grid2(ctx->dev), kBlk2, 0, ctx->stream, ctx->dev, s2, w);
+    else launch_chained(k_coriolis<0, false>, grid2(ctx->dev), kBlk2, 0, ctx->stream, ctx->dev, s2, w);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, (int)e, "coriolis");
   }

@@ -36,6 +36,7 @@ struct I2 {
 // in FP64.
 template <class R3>
 __global__ void k_bf3d(Dev d, Bc3<R3> s) {
+  chain_sync();
   GB_IJ_HALO
   if (i < d.imin || i > d.imax || j < d.jmin || j > d.jmax) return;
   V3<R3> uu{d, s.f3[UU]}, vv{d, s.f3[VV]}, huo{d, s.f3[HUO]}, hvo{d, s.f3[HVO]}, hun{d, s.f3[HUN]}, hvn{d, s.f3[HVN]};
@@ -69,6 +70,7 @@ __global__ void k_bf3d(Dev d, Bc3<R3> s) {
 // i <= imax+1); zz is a scratch 3D array.
 template <class R3>
 __global__ void k_zz(Dev d, Bc3<R3> s, R3* zzp) {
+  chain_sync();
   GB_IJ_HALO
   if (i < d.imin || i > d.imax + 1 || j < d.jmin || j > d.jmax + 1) return;
   I2 az{d, s.az};
@@ -92,6 +94,7 @@ __global__ void k_zz(Dev d, Bc3<R3> s, R3* zzp) {
 constexpr int IPZ_W = 33, IPZ_H = 5;
 template <class R3, bool ZS = false>
 __global__ void k_ip(Dev d, Bc3<R3> s, const R3* zzp) {
+  chain_sync();
   extern __shared__ unsigned char ip_smem[];
   R3* const zsm = reinterpret_cast<R3*>(ip_smem);
   auto zsh = [&](int k, int r, int q) -> R3& { return zsm[(k * IPZ_H + r) * IPZ_W + q]; };
@@ -191,6 +194,7 @@ __global__ void k_ip(Dev d, Bc3<R3> s, const R3* zzp) {
 // columns i = imin..imax+1, j = jmin..jmax+1 with az >= 1.
 template <class R3>
 __global__ void k_zz_lin(Dev d, Bc3<R3> s, R3* zzp) {
+  chain_sync();
   GB_IJ_HALO
   if (i < d.imin || i > d.imax + 1 || j < d.jmin || j > d.jmax + 1) return;
   I2 az{d, s.az};
@@ -228,6 +232,7 @@ __global__ void k_zz_lin(Dev d, Bc3<R3> s, R3* zzp) {
 // 143); its levels below use hvn. Expressions in the reference's order.
 template <class R3>
 __global__ void k_ip_lin(Dev d, Bc3<R3> s, const R3* zzp) {
+  chain_sync();
   GB_IJ_HALO
   V3<R3> hun{d, s.f3[HUN]}, hvn{d, s.f3[HVN]}, buoy{d, s.f3[BUOY]}, idpdx{d, s.f3[IDPDX]}, idpdy{d, s.f3[IDPDY]},
       zz{d, const_cast<R3*>(zzp)};
@@ -394,6 +399,7 @@ static __device__ __forceinline__ int zi_block_max_scan(int v, int* sh) {
 
 template <class R3, int PASS>
 __global__ void __launch_bounds__(128) k_zi_cols(Dev d, Bc3<R3> s, const R3* zzp, ZiScr<R3> z) {
+  chain_sync();
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= z.np) return;
   const int nx = d.imax - d.imin + 1;
@@ -439,6 +445,7 @@ __global__ void __launch_bounds__(128) k_zi_cols(Dev d, Bc3<R3> s, const R3* zzp
 // in-place inclusive max-scan of both key arrays per block of ZI_SCAN positions; block maxima to agg
 static __global__ void __launch_bounds__(ZI_SCAN) k_zi_scan_blocks(int* key_p, int* key_m, int* agg_p, int* agg_m,
                                                             long long np) {
+  chain_sync();
   __shared__ int sh[32];
   const long long p = (long long)blockIdx.x * ZI_SCAN + threadIdx.x;
   int* keys[2] = {key_p, key_m};
@@ -452,6 +459,7 @@ static __global__ void __launch_bounds__(ZI_SCAN) k_zi_scan_blocks(int* key_p, i
 
 // in-place inclusive max-scan of the nb block maxima (one block, chunks of ZI_SCAN)
 static __global__ void __launch_bounds__(ZI_SCAN) k_zi_scan_aggs(int* agg_p, int* agg_m, int nb) {
+  chain_sync();
   __shared__ int sh[32];
   int* aggs[2] = {agg_p, agg_m};
   for (int a = 0; a < 2; ++a) {
@@ -489,6 +497,7 @@ struct SvkWork {
 
 template <class R3>
 __global__ void k_svk_zi(Dev d, Bc3<R3> s, R3* zip) {
+  chain_sync();
   GB_IJ_HALO
   if (i < d.imin || i > d.imax + 1 || j < d.jmin || j > d.jmax + 1) return;
   I2 az{d, s.az};
@@ -594,6 +603,7 @@ __device__ int svk_column(const Dev& d, const Bc3<R3>& s, const R3* zzp, const R
 template <class R3>
 __global__ void __launch_bounds__(128) k_svk_cols(Dev d, Bc3<R3> s, const R3* zzp, const R3* zip, int* flag,
                                                   long long np) {
+  chain_sync();
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= np) return;
   const int nx = d.imax - d.imin + 1;
@@ -611,6 +621,7 @@ __global__ void __launch_bounds__(128) k_svk_cols(Dev d, Bc3<R3> s, const R3* zz
 // the reference's loops in their order with the carried work arrays; only when flagged
 template <class R3>
 __global__ void k_svk_serial(Dev d, Bc3<R3> s, const R3* zzp, const R3* zip, const int* flag) {
+  chain_sync();
   if (*flag == 0) return;
   SvkWork<R3> w;
   for (int k = 0; k <= SVK_KMAX; ++k) {
@@ -632,6 +643,7 @@ __global__ void k_svk_serial(Dev d, Bc3<R3> s, const R3* zzp, const R3* zip, con
 // 1/dx as in the reference (ip_song_wright.F90:128). Expressions in the reference's order.
 template <class R3>
 __global__ void k_ip_sw(Dev d, Bc3<R3> s, const R3* zzp) {
+  chain_sync();
   GB_IJ_HALO
   V3<R3> hn{d, s.f3[HN]}, hun{d, s.f3[HUN]}, hvn{d, s.f3[HVN]}, buoy{d, s.f3[BUOY]}, idpdx{d, s.f3[IDPDX]},
       idpdy{d, s.f3[IDPDY]}, zz{d, const_cast<R3*>(zzp)};
@@ -669,6 +681,7 @@ __global__ void k_ip_sw(Dev d, Bc3<R3> s, const R3* zzp) {
 // the reference. Expressions in the reference's order.
 template <class R3>
 __global__ void k_ip_cf(Dev d, Bc3<R3> s, const R3* zzp) {
+  chain_sync();
   GB_IJ_HALO
   V3<R3> hun{d, s.f3[HUN]}, hvn{d, s.f3[HVN]}, buoy{d, s.f3[BUOY]}, idpdx{d, s.f3[IDPDX]}, idpdy{d, s.f3[IDPDY]},
       zz{d, const_cast<R3*>(zzp)};
@@ -723,6 +736,7 @@ struct SmConst {
 // registers). Expressions in the reference's order.
 template <class R3>
 __global__ void k_sm_cols(Dev d, Bc3<R3> s, R3* zzp, R3* Pp) {
+  chain_sync();
   GB_IJ_HALO
   I2 az{d, s.az};
   V3<R3> hn{d, s.f3[HN]}, buoy{d, s.f3[BUOY]}, zz{d, zzp}, P{d, Pp};
@@ -785,6 +799,7 @@ __global__ void k_sm_cols(Dev d, Bc3<R3> s, R3* zzp, R3* Pp) {
 // order.
 template <class R3>
 __global__ void k_ip_sm(Dev d, Bc3<R3> s, const R3* zzp, const R3* Pp) {
+  chain_sync();
   GB_IJ_HALO
   V3<R3> hun{d, s.f3[HUN]}, hvn{d, s.f3[HVN]}, buoy{d, s.f3[BUOY]}, idpdx{d, s.f3[IDPDX]}, idpdy{d, s.f3[IDPDY]},
       zz{d, const_cast<R3*>(zzp)}, P{d, const_cast<R3*>(Pp)};
@@ -848,6 +863,7 @@ constexpr int UVM_IN = 9;
 constexpr int UVM_THREADS = 128;
 template <class R3, int DIR, bool SM, int NT, int SL = UVM_SLOTS>
 __global__ void __launch_bounds__(NT) k_uvmom3d(Dev d, Bc3<R3> s, R3* RUs, R3* QUs) {
+  chain_sync();
   using T = R3;
   static_assert(SL == 4 || SL == 8, "a ring of 4 or 8 levels");
   __shared__ R3 sl[SL][UVM_IN][NT];
@@ -1029,6 +1045,7 @@ __global__ void __launch_bounds__(NT) k_uvmom3d(Dev d, Bc3<R3> s, R3* RUs, R3* Q
 constexpr int LVC = 64;
 template <class R3>
 __global__ void k_sigma(Dev d, Bc3<R3> s) {
+  chain_sync();
   GB_IJ_HALO
   const int k0 = blockIdx.z * LVC, k1 = min(k0 + LVC, d.kmax + 1);
   V2 sseo{d, s.f2[SSEO]}, ssen{d, s.f2[SSEN]}, H{d, s.f2[HH]}, ssuo{d, s.f2[SSUO]}, ssun{d, s.f2[SSUN]},
@@ -1063,6 +1080,7 @@ __global__ void k_sigma(Dev d, Bc3<R3> s) {
 // stores queue up behind one another).
 template <int N>
 __global__ void __launch_bounds__(128) k_sigma_vec(Dev d, Bc3<float> s) {
+  chain_sync();
   const int ni = d.ni(), nj = d.nj();
   const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * N;
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1118,6 +1136,7 @@ __device__ __forceinline__ R3 sig_h(const Bc3<R3>& s, int e, int hx, long long c
 // k_sigma or uv_advect_3d form no value hold 0.
 template <class R3>
 __global__ void k_col_heights(Dev d, Bc3<R3> s, R3* out) {
+  chain_sync();
   GB_IJ_HALO
   const int ni = d.ni(), nj = d.nj();
   const long long n2 = d.sj * (long long)nj;  // plane pitch (the 2D fields' size)
@@ -1143,6 +1162,7 @@ __global__ void k_col_heights(Dev d, Bc3<R3> s, R3* out) {
 // ww_momentum_3d.F90:74-106 with the layer heights of the column from sig_h (read after k_sigma)
 template <class R3>
 __global__ void k_ww(Dev d, Bc3<R3> s) {
+  chain_sync();
   GB_IJ_HALO
   if (i < d.imin || i > d.imax || j < d.jmin || j > d.jmax) return;
   I2 az{d, s.az};
@@ -1183,6 +1203,7 @@ __global__ void k_ww(Dev d, Bc3<R3> s) {
 template <class R3, int DIR>
 __global__ void k_uvadv3d_prep(Dev d, Bc3<R3> s, R3* fadvp, R3* uuadvp, R3* vvadvp, R3* wwadvp, R3* huadvp,
                                R3* hvadvp) {
+  chain_sync();
   GB_IJ_HALO
   const int k = blockIdx.z;  // one thread per cell and level 0..kmax (independent loads in flight)
   V3<R3> uu{d, s.f3[UU]}, vv{d, s.f3[VV]}, ww{d, s.f3[WW]}, ho{d, s.f3[HO]}, hn{d, s.f3[HN]}, hun{d, s.f3[HUN]},
@@ -1218,6 +1239,7 @@ __global__ void k_uvadv3d_prep(Dev d, Bc3<R3> s, R3* fadvp, R3* uuadvp, R3* vvad
 template <int DIR>
 __global__ void __launch_bounds__(128) k_uvadv3d_prep_vec(Dev d, Bc3<float> s, float* fadvp, float* uuadvp,
                                                         float* vvadvp, float* wwadvp, float* huadvp, float* hvadvp) {
+  chain_sync();
   constexpr int N = 4;
   const int ni = d.ni(), nj = d.nj();
   const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * N;
@@ -1296,6 +1318,7 @@ struct Prep6 {
 template <int N = 4>
 __global__ void __launch_bounds__(128) k_uvadv3d_prep_vec2(Dev d, Bc3<float> s, Prep6 u, Prep6 v,
                                                          const float* colh) {
+  chain_sync();
   const int ni = d.ni(), nj = d.nj();
   const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * N;
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1390,6 +1413,7 @@ __global__ void __launch_bounds__(128) k_uvadv3d_prep_vec2(Dev d, Bc3<float> s, 
 // stresses_3d.F90:50-104 (bottom and surface stresses; FP64 from the bottom layer)
 template <class R3>
 __global__ void k_stresses(Dev d, Bc3<R3> s) {
+  chain_sync();
   GB_IJ_HALO
   V3<R3> uu{d, s.f3[UU]}, vv{d, s.f3[VV]}, hun{d, s.f3[HUN]}, hvn{d, s.f3[HVN]};
   V2 rru{d, s.f2[RRU]}, rrv{d, s.f2[RRV]}, taubx{d, s.f2[TAUBX]}, tauby{d, s.f2[TAUBY]}, taub{d, s.f2[TAUB]},
@@ -1432,6 +1456,7 @@ __device__ __forceinline__ void eos_lin(const Bc3<R3>& s, R3 t, R3 sal, R3& r, R
 // levels 1..kmax over the haloed plane, one thread per cell
 template <class R3>
 __global__ void k_eqstate(Dev d, Bc3<R3> s) {
+  chain_sync();
   GB_IJ_HALO
   const int k = blockIdx.z + 1;
   V3<R3> rho{d, s.f3[RHO]}, buoy{d, s.f3[BUOY]}, T{d, s.f3[TT]}, S{d, s.f3[SS]};
@@ -1444,6 +1469,7 @@ __global__ void k_eqstate(Dev d, Bc3<R3> s) {
 // FP32, 16-byte aligned layouts: 4 consecutive cells per thread with float4 accesses
 template <int N>
 __global__ void __launch_bounds__(128) k_eqstate_vec(Dev d, Bc3<float> s) {
+  chain_sync();
   const int ni = d.ni(), nj = d.nj();
   const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * N;
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1499,6 +1525,7 @@ __device__ __forceinline__ double rho_jackett06(double s, double th) {
 // turbulence closure's buoyancy frequency and are not formed.
 template <class R3, int METHOD>
 __global__ void k_eqstate_nl(Dev d, Bc3<R3> s) {
+  chain_sync();
   GB_IJ_HALO
   const int k = blockIdx.z + 1;
   V3<R3> rho{d, s.f3[RHO]}, buoy{d, s.f3[BUOY]}, T{d, s.f3[TT]}, S{d, s.f3[SS]};
@@ -1527,6 +1554,7 @@ __global__ void k_eqstate_nl(Dev d, Bc3<R3> s) {
 // per column.
 template <class R3>
 __global__ void k_gotm_parabolic(Dev d, Bc3<R3> s) {
+  chain_sync();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + d.imin;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + d.jmin;
   if (i > d.imax || j > d.jmax) return;
@@ -1563,6 +1591,7 @@ __global__ void k_gotm_parabolic(Dev d, Bc3<R3> s) {
 // of the interface under the surface; one thread per column, FP64 arithmetic.
 template <class R3>
 __global__ void k_sw_radiation(Dev d, Bc3<R3> s) {
+  chain_sync();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + d.imin;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + d.jmin;
   if (i > d.imax || j > d.jmax) return;
@@ -1588,6 +1617,7 @@ __global__ void k_sw_radiation(Dev d, Bc3<R3> s) {
 // formed level by level from the bottom up, so no column array is needed.
 template <class R3>
 __global__ void k_temp_source(Dev d, Bc3<R3> s, const R3* __restrict__ S_top, R3* __restrict__ srcp) {
+  chain_sync();
   const int i = blockIdx.x * blockDim.x + threadIdx.x + d.imin;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + d.jmin;
   if (i > d.imax || j > d.jmax) return;
@@ -1624,6 +1654,7 @@ __global__ void k_temp_source(Dev d, Bc3<R3> s, const R3* __restrict__ S_top, R3
 // slow_terms.F90:57-181 (kmax > 1, kumin = kvmin = 1): vertical sums in FP64
 template <class R3>
 __global__ void k_slow_terms(Dev d, Bc3<R3> s) {
+  chain_sync();
   GB_IJ_HALO
   if (i < d.imin || i > d.imax || j < d.jmin || j > d.jmax) return;
   V2 UEx{d, s.f2[UEX]}, VEx{d, s.f2[VEX]}, SlUx{d, s.f2[SLUX]}, SlVx{d, s.f2[SLVX]}, Slru{d, s.f2[SLRU]},
@@ -1659,7 +1690,7 @@ inline dim3 plane_grid(const Dev& d, dim3 blk, int nz = 1) {
 template <class R3>
 int run_col_heights(const Dev& d, cudaStream_t st, const Bc3<R3>& s, R3* out) {
   const dim3 blk(64, 4, 1);
-  k_col_heights<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s, out);
+  launch_chained(k_col_heights<R3>, plane_grid(d, blk), blk, 0, st, d, s, out);
   return (int)cudaGetLastError();
 }
 
@@ -1667,29 +1698,29 @@ template <class R3>
 int run_bc3(int which, const Dev& d, cudaStream_t st, const Bc3<R3>& s, R3* const* scr, const R3* colh) {
   const dim3 blk(32, 4, 1);
   switch (which) {
-    case BC3_BF3D: k_bf3d<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s); break;
-    case BC3_ZZ: k_zz<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s, scr[6]); break;
+    case BC3_BF3D: launch_chained(k_bf3d<R3>, plane_grid(d, blk), blk, 0, st, d, s); break;
+    case BC3_ZZ: launch_chained(k_zz<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6]); break;
     case BC3_IP:
       if constexpr (sizeof(R3) == 4) {  // the interface heights formed in shared memory (no k_zz)
         const size_t dyn = (size_t)(d.kmax + 1) * IPZ_H * IPZ_W * sizeof(R3);
         const cudaError_t e = cudaFuncSetAttribute(k_ip<R3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
         if (e != cudaSuccess) return (int)e;
-        k_ip<R3, true><<<plane_grid(d, blk), blk, dyn, st>>>(d, s, nullptr);
+        launch_chained(k_ip<R3, true>, plane_grid(d, blk), blk, dyn, st, d, s, nullptr);
       } else {
-        k_ip<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s, scr[6]);
+        launch_chained(k_ip<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6]);
       }
       break;
-    case BC3_ZZ_LIN: k_zz_lin<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s, scr[6]); break;
-    case BC3_IP_LIN: k_ip_lin<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s, scr[6]); break;
-    case BC3_IP_SW: k_ip_sw<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s, scr[6]); break;
-    case BC3_IP_CF: k_ip_cf<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s, scr[6]); break;
+    case BC3_ZZ_LIN: launch_chained(k_zz_lin<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6]); break;
+    case BC3_IP_LIN: launch_chained(k_ip_lin<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6]); break;
+    case BC3_IP_SW: launch_chained(k_ip_sw<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6]); break;
+    case BC3_IP_CF: launch_chained(k_ip_cf<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6]); break;
     case BC3_IP_SVK: {  // zz (from k_zz_lin) in scr[6]; zi in scr[5]; the flag in scr[0]
       const long long np = 2LL * (d.imax - d.imin + 1) * (d.jmax - d.jmin + 1);
       int* flag = (int*)scr[0];
       cudaMemsetAsync(flag, 0, sizeof(int), st);
-      k_svk_zi<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s, scr[5]);
-      k_svk_cols<R3><<<(int)((np + 127) / 128), 128, 0, st>>>(d, s, scr[6], scr[5], flag, np);
-      k_svk_serial<R3><<<1, 1, 0, st>>>(d, s, scr[6], scr[5], flag);
+      launch_chained(k_svk_zi<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[5]);
+      launch_chained(k_svk_cols<R3>, (int)((np + 127) / 128), 128, 0, st, d, s, scr[6], scr[5], flag, np);
+      launch_chained(k_svk_serial<R3>, 1, 1, 0, st, d, s, scr[6], scr[5], flag);
       break;
     }
     case BC3_IP_ZI: {  // zz (from k_zz_lin) in scr[6]; the carried-value records in scr[0..5]
@@ -1697,14 +1728,14 @@ int run_bc3(int which, const Dev& d, cudaStream_t st, const Bc3<R3>& s, R3* cons
       const int nb = (int)((np + ZI_SCAN - 1) / ZI_SCAN);
       ZiScr<R3> z{scr[0], scr[4], (int*)scr[1], (int*)scr[5], (int*)scr[2], (int*)scr[3], (int*)scr[3] + nb, np};
       const int g = (int)((np + 127) / 128);
-      k_zi_cols<R3, 1><<<g, 128, 0, st>>>(d, s, scr[6], z);
-      k_zi_scan_blocks<<<nb, ZI_SCAN, 0, st>>>(z.key_p, z.key_m, z.agg_p, z.agg_m, np);
-      k_zi_scan_aggs<<<1, ZI_SCAN, 0, st>>>(z.agg_p, z.agg_m, nb);
-      k_zi_cols<R3, 3><<<g, 128, 0, st>>>(d, s, scr[6], z);
+      launch_chained(k_zi_cols<R3, 1>, g, 128, 0, st, d, s, scr[6], z);
+      launch_chained(k_zi_scan_blocks, nb, ZI_SCAN, 0, st, z.key_p, z.key_m, z.agg_p, z.agg_m, np);
+      launch_chained(k_zi_scan_aggs, 1, ZI_SCAN, 0, st, z.agg_p, z.agg_m, nb);
+      launch_chained(k_zi_cols<R3, 3>, g, 128, 0, st, d, s, scr[6], z);
       break;
     }
-    case BC3_SM_COLS: k_sm_cols<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s, scr[6], scr[0]); break;
-    case BC3_IP_SM: k_ip_sm<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s, scr[6], scr[0]); break;
+    case BC3_SM_COLS: launch_chained(k_sm_cols<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6], scr[0]); break;
+    case BC3_IP_SM: launch_chained(k_ip_sm<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6], scr[0]); break;
     case BC3_UUMOM:
     case BC3_VVMOM: {
       const int nx = d.imax - d.imin + 1, ny = d.jmax - d.jmin + 1;
@@ -1721,7 +1752,7 @@ int run_bc3(int which, const Dev& d, cudaStream_t st, const Bc3<R3>& s, R3* cons
           auto kern = which == BC3_UUMOM ? k_uvmom3d<R3, 0, true, NT, 8> : k_uvmom3d<R3, 1, true, NT, 8>;
           const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
           if (e != cudaSuccess) return (int)e;
-          kern<<<g2, b2, dyn, st>>>(d, s, scr[0], scr[1]);
+          launch_chained(kern, g2, b2, dyn, st, d, s, scr[0], scr[1]);
           done = true;
         }
       }
@@ -1729,9 +1760,9 @@ int run_bc3(int which, const Dev& d, cudaStream_t st, const Bc3<R3>& s, R3* cons
         const dim3 b2(32, 4, 1);
         const dim3 g2((nx + 31) / 32, (ny + 3) / 4, 1);
         if (which == BC3_UUMOM)
-          k_uvmom3d<R3, 0, false, UVM_THREADS><<<g2, b2, 0, st>>>(d, s, scr[0], scr[1]);
+          launch_chained(k_uvmom3d<R3, 0, false, UVM_THREADS>, g2, b2, 0, st, d, s, scr[0], scr[1]);
         else
-          k_uvmom3d<R3, 1, false, UVM_THREADS><<<g2, b2, 0, st>>>(d, s, scr[0], scr[1]);
+          launch_chained(k_uvmom3d<R3, 1, false, UVM_THREADS>, g2, b2, 0, st, d, s, scr[0], scr[1]);
       }
       break;
     }
@@ -1741,14 +1772,14 @@ int run_bc3(int which, const Dev& d, cudaStream_t st, const Bc3<R3>& s, R3* cons
         for (int f : {HO, HN, HUO, HUN, HVO, HVN}) ok = ok && reinterpret_cast<uintptr_t>(s.f3[f]) % 16 == 0;
         if (ok) {
           const dim3 gv((d.ni() + 4 * 32 - 1) / (4 * 32), (d.nj() + 3) / 4, 4);
-          k_sigma_vec<4><<<gv, dim3(32, 4, 1), 0, st>>>(d, s);
+          launch_chained(k_sigma_vec<4>, gv, dim3(32, 4, 1), 0, st, d, s);
           break;
         }
       }
-      k_sigma<R3><<<plane_grid(d, blk, (d.kmax + LVC) / LVC), blk, 0, st>>>(d, s);
+      launch_chained(k_sigma<R3>, plane_grid(d, blk, (d.kmax + LVC) / LVC), blk, 0, st, d, s);
       break;
     }
-    case BC3_WW: k_ww<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s); break;
+    case BC3_WW: launch_chained(k_ww<R3>, plane_grid(d, blk), blk, 0, st, d, s); break;
     case BC3_UVADV_PREP_U:
     case BC3_UVADV_PREP_V: {
       const bool u = which == BC3_UVADV_PREP_U;
@@ -1760,17 +1791,19 @@ int run_bc3(int which, const Dev& d, cudaStream_t st, const Bc3<R3>& s, R3* cons
         if (ok) {
           const dim3 bv(32, 4, 1);
           const dim3 gv((d.ni() + 4 * 32 - 1) / (4 * 32), (d.nj() + 3) / 4, d.kmax + 1);
-          if (u) k_uvadv3d_prep_vec<0><<<gv, bv, 0, st>>>(d, s, scr[0], scr[1], scr[2], scr[3], scr[4], scr[5]);
-          else k_uvadv3d_prep_vec<1><<<gv, bv, 0, st>>>(d, s, scr[0], scr[1], scr[2], scr[3], scr[4], scr[5]);
+          if (u) launch_chained(k_uvadv3d_prep_vec<0>, gv, bv, 0, st, d, s, scr[0], scr[1], scr[2], scr[3], scr[4],
+                                scr[5]);
+          else launch_chained(k_uvadv3d_prep_vec<1>, gv, bv, 0, st, d, s, scr[0], scr[1], scr[2], scr[3], scr[4],
+                              scr[5]);
           break;
         }
       }
       if (u)
-        k_uvadv3d_prep<R3, 0><<<plane_grid(d, blk, d.kmax + 1), blk, 0, st>>>(d, s, scr[0], scr[1], scr[2], scr[3],
-                                                                              scr[4], scr[5]);
+        launch_chained(k_uvadv3d_prep<R3, 0>, plane_grid(d, blk, d.kmax + 1), blk, 0, st, d, s, scr[0], scr[1],
+                       scr[2], scr[3], scr[4], scr[5]);
       else
-        k_uvadv3d_prep<R3, 1><<<plane_grid(d, blk, d.kmax + 1), blk, 0, st>>>(d, s, scr[0], scr[1], scr[2], scr[3],
-                                                                              scr[4], scr[5]);
+        launch_chained(k_uvadv3d_prep<R3, 1>, plane_grid(d, blk, d.kmax + 1), blk, 0, st, d, s, scr[0], scr[1],
+                       scr[2], scr[3], scr[4], scr[5]);
       break;
     }
     case BC3_UVADV_PREP_UV: {  // FP32 only: U grid into scr[0..5], V grid into scr[7..12]
@@ -1783,36 +1816,35 @@ int run_bc3(int which, const Dev& d, cudaStream_t st, const Bc3<R3>& s, R3* cons
         if (ok) {
           const dim3 bv(32, 4, 1);
           const dim3 gv((d.ni() + 4 * 32 - 1) / (4 * 32), (d.nj() + 3) / 4, d.kmax + 1);
-          k_uvadv3d_prep_vec2<4><<<gv, bv, 0, st>>>(d, s, Prep6{{scr[0], scr[1], scr[2], scr[3], scr[4], scr[5]}},
-                                                    Prep6{{scr[7], scr[8], scr[9], scr[10], scr[11], scr[12]}},
-                                                    colh);
+          launch_chained(k_uvadv3d_prep_vec2<4>, gv, bv, 0, st, d, s, Prep6{{scr[0], scr[1], scr[2], scr[3], scr[4],
+                         scr[5]}}, Prep6{{scr[7], scr[8], scr[9], scr[10], scr[11], scr[12]}}, colh);
         } else {
-          k_uvadv3d_prep<R3, 0><<<plane_grid(d, blk, d.kmax + 1), blk, 0, st>>>(d, s, scr[0], scr[1], scr[2],
-                                                                                scr[3], scr[4], scr[5]);
-          k_uvadv3d_prep<R3, 1><<<plane_grid(d, blk, d.kmax + 1), blk, 0, st>>>(d, s, scr[7], scr[8], scr[9],
-                                                                                scr[10], scr[11], scr[12]);
+          launch_chained(k_uvadv3d_prep<R3, 0>, plane_grid(d, blk, d.kmax + 1), blk, 0, st, d, s, scr[0], scr[1],
+                         scr[2], scr[3], scr[4], scr[5]);
+          launch_chained(k_uvadv3d_prep<R3, 1>, plane_grid(d, blk, d.kmax + 1), blk, 0, st, d, s, scr[7], scr[8],
+                         scr[9], scr[10], scr[11], scr[12]);
         }
         break;
       } else {
         return (int)cudaErrorInvalidValue;
       }
     }
-    case BC3_STRESSES: k_stresses<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s); break;
-    case BC3_EQSTATE_UNESCO: k_eqstate_nl<R3, 2><<<plane_grid(d, blk, d.kmax), blk, 0, st>>>(d, s); break;
-    case BC3_EQSTATE_JACKETT: k_eqstate_nl<R3, 3><<<plane_grid(d, blk, d.kmax), blk, 0, st>>>(d, s); break;
+    case BC3_STRESSES: launch_chained(k_stresses<R3>, plane_grid(d, blk), blk, 0, st, d, s); break;
+    case BC3_EQSTATE_UNESCO: launch_chained(k_eqstate_nl<R3, 2>, plane_grid(d, blk, d.kmax), blk, 0, st, d, s); break;
+    case BC3_EQSTATE_JACKETT: launch_chained(k_eqstate_nl<R3, 3>, plane_grid(d, blk, d.kmax), blk, 0, st, d, s); break;
     case BC3_GOTM_PARABOLIC: {
       const dim3 g((d.imax - d.imin + 1 + 31) / 32, (d.jmax - d.jmin + 1 + 3) / 4, 1);
-      k_gotm_parabolic<R3><<<g, blk, 0, st>>>(d, s);
+      launch_chained(k_gotm_parabolic<R3>, g, blk, 0, st, d, s);
       break;
     }
     case BC3_SW_RADIATION: {
       const dim3 g((d.imax - d.imin + 1 + 31) / 32, (d.jmax - d.jmin + 1 + 3) / 4, 1);
-      k_sw_radiation<R3><<<g, blk, 0, st>>>(d, s);
+      launch_chained(k_sw_radiation<R3>, g, blk, 0, st, d, s);
       break;
     }
     case BC3_TEMP_SOURCE: {  // scr[0] = the source array, scr[1] = the top-level salinity (may be null)
       const dim3 g((d.imax - d.imin + 1 + 31) / 32, (d.jmax - d.jmin + 1 + 3) / 4, 1);
-      k_temp_source<R3><<<g, blk, 0, st>>>(d, s, scr[1], scr[0]);
+      launch_chained(k_temp_source<R3>, g, blk, 0, st, d, s, scr[1], scr[0]);
       break;
     }
     case BC3_EQSTATE: {
@@ -1821,14 +1853,14 @@ int run_bc3(int which, const Dev& d, cudaStream_t st, const Bc3<R3>& s, R3* cons
         for (int f : {TT, SS, RHO, BUOY}) ok = ok && reinterpret_cast<uintptr_t>(s.f3[f]) % 16 == 0;
         if (ok) {
           const dim3 gv((d.ni() + 4 * 32 - 1) / (4 * 32), (d.nj() + 3) / 4, d.kmax);
-          k_eqstate_vec<4><<<gv, dim3(32, 4, 1), 0, st>>>(d, s);
+          launch_chained(k_eqstate_vec<4>, gv, dim3(32, 4, 1), 0, st, d, s);
           break;
         }
       }
-      k_eqstate<R3><<<plane_grid(d, blk, d.kmax), blk, 0, st>>>(d, s);
+      launch_chained(k_eqstate<R3>, plane_grid(d, blk, d.kmax), blk, 0, st, d, s);
       break;
     }
-    case BC3_SLOW_TERMS: k_slow_terms<R3><<<plane_grid(d, blk), blk, 0, st>>>(d, s); break;
+    case BC3_SLOW_TERMS: launch_chained(k_slow_terms<R3>, plane_grid(d, blk), blk, 0, st, d, s); break;
     default: return (int)cudaErrorInvalidValue;
   }
   return (int)cudaGetLastError();

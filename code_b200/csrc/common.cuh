@@ -30,6 +30,29 @@ inline Dev to_dev(const getm_domain& d) {
   return v;
 }
 
+// Programmatic dependent launch for the chains of kernels of a step: a kernel launched by
+// launch_chained is set up while its predecessor in the stream still runs, and every one of its
+// threads calls chain_sync() before it touches memory, which waits until that one, and with it every
+// kernel before, has completed with its writes visible. No kernel lets its successor start early: the
+// waiting blocks would take its place on the SMs (barotropic 128 x 96, 20 micro steps: 783 us with plain
+// launches, 617 with the successor released at the start, 556 released by completion; 2048x2048x50
+// mixed step 33.3, 34.8, 33.1 ms). A kernel launched the plain way passes through chain_sync().
+__device__ __forceinline__ void chain_sync() { cudaGridDependencySynchronize(); }
+template <class... P, class... A>
+inline int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = at;
+  c.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // Scheme ids (advection.F90:60-62)
 enum : int { NOADV = 0, UPSTREAM = 1, UPSTREAM_2DH = 2, P2 = 3, SUPERBEE = 4, MUSCL = 5, P2_PDM = 6 };
 

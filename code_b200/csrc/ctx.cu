@@ -28,6 +28,7 @@ bool fp32_micro_steps_enabled() { return g_fp32_micro.load(std::memory_order_rel
 // init_advection (advection.F90:263-318) from az/au/av/ax.
 __global__ void k_build_masks(Dev d, const int32_t* __restrict__ az, const int32_t* __restrict__ au,
                               const int32_t* __restrict__ av, const int32_t* __restrict__ ax, uint8_t* planes) {
+  chain_sync();
   const int ii = blockIdx.x * blockDim.x + threadIdx.x;
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
   const int ni = d.ni(), nj = d.nj();
@@ -57,7 +58,7 @@ int run_build_masks(const Dev& d, cudaStream_t s, const int32_t* az, const int32
                     const int32_t* ax, uint8_t* planes) {
   dim3 blk(64, 4, 1);
   dim3 grd((d.ni() + 63) / 64, (d.nj() + 3) / 4, 1);
-  k_build_masks<<<grd, blk, 0, s>>>(d, az, au, av, ax, planes);
+  launch_chained(k_build_masks, grd, blk, 0, s, d, az, au, av, ax, planes);
   return (int)cudaGetLastError();
 }
 
@@ -450,6 +451,7 @@ namespace gb {
 template <class W>
 __global__ void k_rows_copy(const Dev d, char* f, char* buf, int r0, int nrows, int nk, int words_per_row,
                             long long row_stride_w, long long level_stride_w, int to_buf) {
+  chain_sync();
   const long long n = (long long)words_per_row * nrows * nk;
   W* fw = reinterpret_cast<W*>(f);
   W* bw = reinterpret_cast<W*>(buf);
@@ -482,14 +484,14 @@ static int rows_copy(getm_ctx* ctx, void* f, int elem_bytes, int nk, int j_first
   char* fc = static_cast<char*>(f);
   char* bc = static_cast<char*>(buf);
   if (wb == 16)
-    k_rows_copy<int4><<<blocks, 256, 0, ctx->stream>>>(d, fc, bc, r0, nrows, nk, (int)(row_bytes / 16), sj_b / 16,
-                                                       sk_b / 16, to_buf);
+    launch_chained(k_rows_copy<int4>, blocks, 256, 0, ctx->stream, d, fc, bc, r0, nrows, nk, (int)(row_bytes / 16),
+                   sj_b / 16, sk_b / 16, to_buf);
   else if (wb == 8)
-    k_rows_copy<long long><<<blocks, 256, 0, ctx->stream>>>(d, fc, bc, r0, nrows, nk, (int)(row_bytes / 8), sj_b / 8,
-                                                            sk_b / 8, to_buf);
+    launch_chained(k_rows_copy<long long>, blocks, 256, 0, ctx->stream, d, fc, bc, r0, nrows, nk,
+                   (int)(row_bytes / 8), sj_b / 8, sk_b / 8, to_buf);
   else
-    k_rows_copy<int><<<blocks, 256, 0, ctx->stream>>>(d, fc, bc, r0, nrows, nk, (int)(row_bytes / 4), sj_b / 4,
-                                                      sk_b / 4, to_buf);
+    launch_chained(k_rows_copy<int>, blocks, 256, 0, ctx->stream, d, fc, bc, r0, nrows, nk, (int)(row_bytes / 4),
+                   sj_b / 4, sk_b / 4, to_buf);
   GB_TRY(cudaGetLastError(), "halo rows");
   return GETM_OK;
 }

@@ -386,6 +386,7 @@ __global__ void __launch_bounds__(TU, sizeof(R) == 4 ? 16 : 8) k_sweep_u_tile(De
                                                      const R* __restrict__ U, const R* __restrict__ DU,
                                                      const uint8_t* __restrict__ mflux,
                                                      const uint8_t* __restrict__ mupd, uint8_t* code) {
+  chain_sync();
   __shared__ R sf[2][NF][TU + 3];   // f(i0-2 .. i0+TU)
   __shared__ R sU[2][TU];           // U(i0-1 .. i0+TU-2)
   __shared__ R sDU[2][TU];
@@ -519,6 +520,7 @@ __global__ void __launch_bounds__(TVX * TVY, sizeof(R) == 4 ? (NF == 1 ? 8 : 6) 
     k_sweep_v_tile(Dev d, SweepC<R> C, int nk, TracerSet<R, NF> F, const R* Di_src, R* Di_dst, R* adv,
                    const R* __restrict__ V, const R* __restrict__ DV, const uint8_t* __restrict__ mflux,
                    const uint8_t* __restrict__ mupd, uint8_t* code) {
+  chain_sync();
   __shared__ R sf[2][NF][TVY + 4][TVX];  // f(j0-2 .. j0+TVY+1)
   __shared__ R sV[2][TVY + 1][TVX];      // V(j0-1 .. j0+TVY-1)
   __shared__ R sDV[2][TVY + 1][TVX];
@@ -688,6 +690,7 @@ __global__ void __launch_bounds__(128) k_sweep_w(Dev d, R dt, R splitfac, int ks
                                                  const R* f, const R* fi_src, R* fi_dst, R* hi, R* adv,
                                                  const R* __restrict__ ww,
                                                  const int32_t* __restrict__ az, uint8_t* code, __half* lo = nullptr) {
+  chain_sync();
   const int ii = blockIdx.x * blockDim.x + threadIdx.x;
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
   // columns i = imin-2..imax+1, j = jmin-2..jmax+1 (adv_split_w.F90:160-162)
@@ -758,6 +761,7 @@ template <class R, int S>
 __global__ void __launch_bounds__(128) k_sweep_w2(Dev d, R dt, R splitfac, R* fa, R* fb, R* hi,
                                                   const R* __restrict__ ww, const int32_t* __restrict__ az,
                                                   __half* lo_a = nullptr, __half* lo_b = nullptr) {
+  chain_sync();
   const int ii = blockIdx.x * blockDim.x + threadIdx.x;
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
   if (ii >= d.ni() - 1 || jj >= d.nj() - 1) return;
@@ -829,6 +833,7 @@ __global__ void __launch_bounds__(64) k_sweep_w_iter(Dev d, R dt, R splitfac, in
                                                      const R* __restrict__ ww,
                                                      const int32_t* __restrict__ az,
                                                      unsigned long long* warn, __half* lo = nullptr) {
+  chain_sync();
   const int ii = blockIdx.x * blockDim.x + threadIdx.x;
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
   if (ii >= d.ni() - 1 || jj >= d.nj() - 1) return;
@@ -956,6 +961,7 @@ template <class R, int NF, bool IL = false>
 __global__ void __launch_bounds__(128) k_vdiff(Dev d, R dt, R cnpar, VdSet<R, NF> F, const R* __restrict__ hn,
                                                const R* __restrict__ nuh, const int32_t* __restrict__ az,
                                                long long hsk) {
+  chain_sync();
   const int kmax = d.kmax;
   const int i = d.imin + blockIdx.x * blockDim.x + threadIdx.x;
   const int j = d.jmin + blockIdx.y * blockDim.y + threadIdx.y;
@@ -1158,6 +1164,7 @@ template <class R>
 __global__ void __launch_bounds__(TRN) k_tridiag(int ncol, int kmax, int fi, int lt, const R* __restrict__ au,
                                                  const R* __restrict__ bu, const R* __restrict__ cu,
                                                  const R* __restrict__ du, R* value) {
+  chain_sync();
   extern __shared__ unsigned char smem_raw[];
   R* const ru_s = reinterpret_cast<R*>(smem_raw) + threadIdx.x;
   R* const qu_s = ru_s + (kmax + 1) * TRN;
@@ -1218,6 +1225,7 @@ __global__ void __launch_bounds__(TRN) k_tridiag(int ncol, int kmax, int fi, int
 template <class R>
 __global__ void k_finalise(Dev d, R dt, R* f, const R* __restrict__ ho, const R* __restrict__ adv,
                            const R* __restrict__ hi, const uint8_t* __restrict__ mfin) {
+  chain_sync();
   const int ii = blockIdx.x * blockDim.x + threadIdx.x;
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
   if (ii >= d.ni() || jj >= d.nj()) return;
@@ -1248,6 +1256,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_content_partial(Dev d, const R*
                                                                  const R* __restrict__ h,
                                                                  const int32_t* __restrict__ az,
                                                                  double* partial) {
+  chain_sync();
   __shared__ Neu sh[RED_THREADS];
   const int nx = d.imax - d.imin + 1, ny = d.jmax - d.jmin + 1;
   const long long ncell = (long long)nx * ny * d.kmax;
@@ -1278,6 +1287,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_content_partial(Dev d, const R*
 
 static __global__ void __launch_bounds__(RED_THREADS) k_content_final(const double* partial, int nb,
                                                                         double* out) {
+  chain_sync();
   __shared__ Neu sh[RED_THREADS];
   Neu acc{0.0, 0.0};
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
@@ -1299,6 +1309,7 @@ static __global__ void __launch_bounds__(RED_THREADS) k_content_final(const doub
 template <class R>
 __global__ void k_check_range(Dev d, const R* __restrict__ f, const int32_t* __restrict__ az, R lo, R hi,
                               unsigned long long* count) {
+  chain_sync();
   const int ii = blockIdx.x * blockDim.x + threadIdx.x;
   const int jj = blockIdx.y * blockDim.y + threadIdx.y;
   const int nx = d.imax - d.imin + 1, ny = d.jmax - d.jmin + 1;

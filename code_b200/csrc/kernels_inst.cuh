@@ -82,11 +82,11 @@ int run_sweep_h(const Dev& d, cudaStream_t s, int nk, R dt, R splitfac, int sche
           SweepC<R> Cu = C;
           Cu.adv_init = adv_init && adv ? 1 : 0;
           if (comp)
-            k_sweep_u_vec<R, S, REC, NF, true><<<grd, blk, 0, s>>>(d, Cu, nk, set, Di_src, Di_dst, adv, U, DU,
-                                                                   mflux, mupd, code);
+            launch_chained(k_sweep_u_vec<R, S, REC, NF, true>, grd, blk, 0, s, d, Cu, nk, set, Di_src, Di_dst, adv, U,
+                           DU, mflux, mupd, code);
           else
-            k_sweep_u_vec<R, S, REC, NF, false><<<grd, blk, 0, s>>>(d, Cu, nk, set, Di_src, Di_dst, adv, U, DU,
-                                                                    mflux, mupd, code);
+            launch_chained(k_sweep_u_vec<R, S, REC, NF, false>, grd, blk, 0, s, d, Cu, nk, set, Di_src, Di_dst, adv,
+                           U, DU, mflux, mupd, code);
           return (int)cudaGetLastError();
         }
         if (vec) {
@@ -99,11 +99,11 @@ int run_sweep_h(const Dev& d, cudaStream_t s, int nk, R dt, R splitfac, int sche
             dim3 blk(32, VKW, 1);
             dim3 grd((unsigned)nx, (d.nj() + rows - 1) / rows, (unsigned)nz);
             if (comp)
-              k_sweep_v_vec<R, S, REC, NF, VN, true><<<grd, blk, 0, s>>>(d, C, nk, rows, set, Di_src, Di_dst, adv,
-                                                                         U, DU, mflux, mupd, code);
+              launch_chained(k_sweep_v_vec<R, S, REC, NF, VN, true>, grd, blk, 0, s, d, C, nk, rows, set, Di_src,
+                             Di_dst, adv, U, DU, mflux, mupd, code);
             else
-              k_sweep_v_vec<R, S, REC, NF, VN, false><<<grd, blk, 0, s>>>(d, C, nk, rows, set, Di_src, Di_dst, adv,
-                                                                          U, DU, mflux, mupd, code);
+              launch_chained(k_sweep_v_vec<R, S, REC, NF, VN, false>, grd, blk, 0, s, d, C, nk, rows, set, Di_src,
+                             Di_dst, adv, U, DU, mflux, mupd, code);
             return (int)cudaGetLastError();
           };
           // float4 lanes for one field; float2 lanes for a tracer pair (72 registers against 116:
@@ -121,20 +121,20 @@ int run_sweep_h(const Dev& d, cudaStream_t s, int nk, R dt, R splitfac, int sche
           while (rows > 8 && nx * ((d.nj() + rows - 1) / rows) * nz * VKW < 148LL * 24) rows /= 2;
           dim3 blk(32, VKW, 1);
           dim3 grd((unsigned)nx, (d.nj() + rows - 1) / rows, (unsigned)nz);
-          k_sweep_v_vec<R, S, REC, NF, VN><<<grd, blk, 0, s>>>(d, C, nk, rows, set, Di_src, Di_dst, adv, U, DU,
-                                                               mflux, mupd, code);
+          launch_chained(k_sweep_v_vec<R, S, REC, NF, VN>, grd, blk, 0, s, d, C, nk, rows, set, Di_src, Di_dst, adv,
+                         U, DU, mflux, mupd, code);
           return (int)cudaGetLastError();
         }
       }
       if (DIR == 0) {
         dim3 grd((d.ni() + OWU - 1) / OWU, d.nj(), nz);
-        k_sweep_u_tile<R, S, REC, NF><<<grd, TU, 0, s>>>(d, C, nk, set, Di_src, Di_dst, adv, U, DU, mflux, mupd,
-                                                         code);
+        launch_chained(k_sweep_u_tile<R, S, REC, NF>, grd, TU, 0, s, d, C, nk, set, Di_src, Di_dst, adv, U, DU, mflux,
+                       mupd, code);
       } else {
         dim3 blk(TVX, TVY, 1);
         dim3 grd((d.ni() + TVX - 1) / TVX, (d.nj() + TVY - 1) / TVY, nz);
-        k_sweep_v_tile<R, S, REC, NF><<<grd, blk, 0, s>>>(d, C, nk, set, Di_src, Di_dst, adv, U, DU, mflux, mupd,
-                                                          code);
+        launch_chained(k_sweep_v_tile<R, S, REC, NF>, grd, blk, 0, s, d, C, nk, set, Di_src, Di_dst, adv, U, DU,
+                       mflux, mupd, code);
       }
       return (int)cudaGetLastError();
     };
@@ -201,8 +201,8 @@ int run_adv_pass(const Dev& d, cudaStream_t s, bool vu, int nk, R dt, int scheme
       int rows = 64;
       while (rows > 8 && strips * ((d.nj() + rows - 1) / rows) * nk < 148LL * 12) rows /= 2;
       const dim3 blk(32, AW, 1), grd((unsigned)strips, (unsigned)((d.nj() + rows * AW - 1) / (rows * AW)), (unsigned)nk);
-      if (vu) k_adv_vu<R, S, REC, NF, N, LO, MOM><<<grd, blk, 0, s>>>(d, C, F, rows);
-      else k_adv_uv<R, S, REC, NF, N, LO, MOM><<<grd, blk, 0, s>>>(d, C, F, rows);
+      if (vu) launch_chained(k_adv_vu<R, S, REC, NF, N, LO, MOM>, grd, blk, 0, s, d, C, F, rows);
+      else launch_chained(k_adv_uv<R, S, REC, NF, N, LO, MOM>, grd, blk, 0, s, d, C, F, rows);
       return (int)cudaGetLastError();
     };
     using std::integral_constant;
@@ -241,7 +241,7 @@ int run_sweep_w2(const Dev& d, cudaStream_t s, R dt, R splitfac, int scheme, R* 
     constexpr int S = decltype(sc)::value;
     dim3 blk(64, 2, 1);
     dim3 grd((d.ni() - 1 + blk.x - 1) / blk.x, (d.nj() - 1 + blk.y - 1) / blk.y, 1);
-    k_sweep_w2<R, S><<<grd, blk, 0, s>>>(d, dt, splitfac, fa, fb, hi, ww, az, lo_a, lo_b);
+    launch_chained(k_sweep_w2<R, S>, grd, blk, 0, s, d, dt, splitfac, fa, fb, hi, ww, az, lo_a, lo_b);
     return (int)cudaGetLastError();
   });
 }
@@ -255,8 +255,8 @@ int run_sweep_w(const Dev& d, cudaStream_t s, R dt, R splitfac, int scheme, int 
     if (code || mom) return (int)cudaErrorInvalidValue;
     dim3 blk(32, 2, 1);
     dim3 grd((d.ni() - 1 + blk.x - 1) / blk.x, (d.nj() - 1 + blk.y - 1) / blk.y, 1);
-    k_sweep_w_iter<R><<<grd, blk, 0, s>>>(d, dt, splitfac, scheme, kshift, itersmax, f, fi_src, fi_dst, hi,
-                                          adv, ww, az, warn, lo);
+    launch_chained(k_sweep_w_iter<R>, grd, blk, 0, s, d, dt, splitfac, scheme, kshift, itersmax, f, fi_src, fi_dst,
+                   hi, adv, ww, az, warn, lo);
     return (int)cudaGetLastError();
   }
   return dispatch_scheme(scheme, [&](auto sc) {
@@ -264,17 +264,17 @@ int run_sweep_w(const Dev& d, cudaStream_t s, R dt, R splitfac, int scheme, int 
     dim3 blk(64, 2, 1);
     dim3 grd((d.ni() - 1 + blk.x - 1) / blk.x, (d.nj() - 1 + blk.y - 1) / blk.y, 1);
     if (code)
-      k_sweep_w<R, S, true><<<grd, blk, 0, s>>>(d, dt, splitfac, kshift, f, fi_src, fi_dst, hi, adv, ww, az, code,
-                                                lo);
+      launch_chained(k_sweep_w<R, S, true>, grd, blk, 0, s, d, dt, splitfac, kshift, f, fi_src, fi_dst, hi, adv, ww,
+                     az, code, lo);
     else if (mom == 1)
-      k_sweep_w<R, S, false, 1><<<grd, blk, 0, s>>>(d, dt, splitfac, kshift, f, fi_src, fi_dst, hi, adv, ww, az,
-                                                    nullptr, lo);
+      launch_chained(k_sweep_w<R, S, false, 1>, grd, blk, 0, s, d, dt, splitfac, kshift, f, fi_src, fi_dst, hi, adv,
+                     ww, az, nullptr, lo);
     else if (mom == 2)
-      k_sweep_w<R, S, false, 2><<<grd, blk, 0, s>>>(d, dt, splitfac, kshift, f, fi_src, fi_dst, hi, adv, ww, az,
-                                                    nullptr, lo);
+      launch_chained(k_sweep_w<R, S, false, 2>, grd, blk, 0, s, d, dt, splitfac, kshift, f, fi_src, fi_dst, hi, adv,
+                     ww, az, nullptr, lo);
     else
-      k_sweep_w<R, S, false><<<grd, blk, 0, s>>>(d, dt, splitfac, kshift, f, fi_src, fi_dst, hi, adv, ww, az,
-                                                 nullptr, lo);
+      launch_chained(k_sweep_w<R, S, false>, grd, blk, 0, s, d, dt, splitfac, kshift, f, fi_src, fi_dst, hi, adv, ww,
+                     az, nullptr, lo);
     return (int)cudaGetLastError();
   });
 }
@@ -284,7 +284,7 @@ int run_finalise(const Dev& d, cudaStream_t s, R dt, R* f, const R* ho, const R*
                  const uint8_t* mfin) {
   dim3 blk(64, 4, 1);
   dim3 grd((d.ni() + blk.x - 1) / blk.x, (d.nj() + blk.y - 1) / blk.y, d.kmax);
-  k_finalise<R><<<grd, blk, 0, s>>>(d, dt, f, ho, adv, hi, mfin);
+  launch_chained(k_finalise<R>, grd, blk, 0, s, d, dt, f, ho, adv, hi, mfin);
   return (int)cudaGetLastError();
 }
 
@@ -297,7 +297,7 @@ int run_vdiff(const Dev& d, cudaStream_t s, R dt, R cnpar, R avmol, R* S, const 
   dim3 blk(32, 4, 1);
   dim3 grd((nx + 31) / 32, (ny + 3) / 4, 1);
   VdSet<R, 1> F{{{Sin ? Sin : S, S, src, rus, qus, S2, lo, avmol}}};
-  k_vdiff<R, 1><<<grd, blk, 0, s>>>(d, dt, cnpar, F, hn, nuh, az, d.sk);
+  launch_chained(k_vdiff<R, 1>, grd, blk, 0, s, d, dt, cnpar, F, hn, nuh, az, d.sk);
   return (int)cudaGetLastError();
 }
 
@@ -315,9 +315,9 @@ int run_vdiff2(const Dev& d, cudaStream_t s, R dt, R cnpar, const R* hn, const R
   // qus_a == qus_b == nullptr: each tracer's (ru, qu) pairs interleaved in its rus array (two
   // elements per cell): one access per level instead of two
   if (!qus_a && !qus_b)
-    k_vdiff<R, 2, true><<<grd, blk, 0, s>>>(d, dt, cnpar, F, hn, nuh, az, hn2d ? 0LL : d.sk);
+    launch_chained(k_vdiff<R, 2, true>, grd, blk, 0, s, d, dt, cnpar, F, hn, nuh, az, hn2d ? 0LL : d.sk);
   else
-    k_vdiff<R, 2><<<grd, blk, 0, s>>>(d, dt, cnpar, F, hn, nuh, az, hn2d ? 0LL : d.sk);
+    launch_chained(k_vdiff<R, 2>, grd, blk, 0, s, d, dt, cnpar, F, hn, nuh, az, hn2d ? 0LL : d.sk);
   return (int)cudaGetLastError();
 }
 
@@ -329,15 +329,15 @@ int run_tridiag(cudaStream_t s, int ncol, int kmax, int fi, int lt, const R* au,
     const cudaError_t e = cudaFuncSetAttribute(k_tridiag<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  k_tridiag<R><<<(ncol + TRN - 1) / TRN, TRN, smem, s>>>(ncol, kmax, fi, lt, au, bu, cu, du, value);
+  launch_chained(k_tridiag<R>, (ncol + TRN - 1) / TRN, TRN, smem, s, ncol, kmax, fi, lt, au, bu, cu, du, value);
   return (int)cudaGetLastError();
 }
 
 template <class R>
 int run_content(const Dev& d, cudaStream_t s, const R* f, const R* h, const int32_t* az, double* partial,
                 double* out) {
-  k_content_partial<R><<<RED_BLOCKS, RED_THREADS, 0, s>>>(d, f, h, az, partial);
-  k_content_final<<<1, RED_THREADS, 0, s>>>(partial, RED_BLOCKS, out);
+  launch_chained(k_content_partial<R>, RED_BLOCKS, RED_THREADS, 0, s, d, f, h, az, partial);
+  launch_chained(k_content_final, 1, RED_THREADS, 0, s, partial, RED_BLOCKS, out);
   return (int)cudaGetLastError();
 }
 
@@ -347,7 +347,7 @@ int run_check_range(const Dev& d, cudaStream_t s, const R* f, const int32_t* az,
   dim3 blk(64, 4, 1);
   const int nx = d.imax - d.imin + 1, ny = d.jmax - d.jmin + 1;
   dim3 grd((nx + blk.x - 1) / blk.x, (ny + blk.y - 1) / blk.y, 1);
-  k_check_range<R><<<grd, blk, 0, s>>>(d, f, az, lo, hi, count);
+  launch_chained(k_check_range<R>, grd, blk, 0, s, d, f, az, lo, hi, count);
   return (int)cudaGetLastError();
 }
 

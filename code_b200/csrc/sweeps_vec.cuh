@@ -191,6 +191,7 @@ __global__ void __launch_bounds__(32 * VKW) k_sweep_v_vec(Dev d, SweepC<R> C, in
                                                         const R* __restrict__ V, const R* __restrict__ DV,
                                                         const uint8_t* __restrict__ mflux,
                                                         const uint8_t* __restrict__ mupd, uint8_t* code) {
+  chain_sync();
   constexpr int N = VN;
   constexpr int VB = N * (int)sizeof(R);
   // slots: f(j+2) per field; for a single field also fi(j) and adv(j) (a tracer pair reads fi
@@ -405,6 +406,7 @@ __global__ void __launch_bounds__(32 * UWB) k_sweep_u_vec(Dev d, SweepC<R> C, in
                                                         const R* __restrict__ U, const R* __restrict__ DU,
                                                         const uint8_t* __restrict__ mflux,
                                                         const uint8_t* __restrict__ mupd, uint8_t* code) {
+  chain_sync();
   constexpr int N = 16 / sizeof(R);
   // slots: f per field; for a single field also fi and adv; U, DU, Di
   constexpr int XU = NF == 1 ? 2 : NF, XDU = XU + 1, XDI = XU + 2, XAD = XU + 3;
