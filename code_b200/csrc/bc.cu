@@ -1580,7 +1580,7 @@ int bc3(getm_ctx* ctx, const getm_bc_state* st, int which, int slot, unsigned sk
 }
 
 // do_internal_pressure (internal_pressure.F90:181-274) with the configured method (check_state
-// admits 1 to 7): heights of the layer interfaces (1, 5) or of the pressure points (2, 3, 4, 7; 6
+// admits 1 to 7): heights of the layer interfaces (5; 1 forms its own) or of the pressure points (2, 3, 4, 7; 6
 // over the whole haloed domain, with its column integrals), then the gradients idpdx, idpdy
 template <class R3>
 int internal_pressure(getm_ctx* ctx, const getm_bc_state* st) {
@@ -1594,8 +1594,7 @@ int internal_pressure(getm_ctx* ctx, const getm_bc_state* st) {
                   : ipm == 5 ? BC3_IP_CF
                              : BC3_IP_SM;
   int rc;
-  // the FP32 Blumberg-Mellor integral forms its interface heights itself (k_ip with ZS)
-  const bool zz_inside = sizeof(R3) == 4 && ipm == 1;
+  const bool zz_inside = ipm == 1;  // the Blumberg-Mellor integral forms its interface heights itself
   if (!zz_inside &&
       (rc = bc3<R3>(ctx, st, ipm == 6 ? BC3_SM_COLS : centres ? BC3_ZZ_LIN : BC3_ZZ, GETM_TIM_BC3D)))
     return rc;

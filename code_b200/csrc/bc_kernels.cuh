@@ -87,56 +87,53 @@ __global__ void k_zz(Dev d, Bc3<R3> s, R3* zzp) {
   }
 }
 
-// ip_blumberg_mellor.F90:94-148: downward integral of the buoyancy gradient per U and V column.
-// ZS (blocks of 32 x 4 points): the interface heights of the block's columns and of the next column
-// and row (the neighbours across the faces) are formed into dynamic shared memory with k_zz's
-// expressions, (kmax+1) x 5 x 33 values, instead of read from the zz array that k_zz writes.
-constexpr int IPZ_W = 33, IPZ_H = 5;
-template <class R3, bool ZS = false>
-__global__ void k_ip(Dev d, Bc3<R3> s, const R3* zzp) {
+// ip_blumberg_mellor.F90:83-148: interface heights and downward integral of the buoyancy gradient per U
+// and V column. One thread per point, its U and V columns side by side: the integrals share the
+// point's buoyancy and heights. Bound by memory latency (one read, two writes per level), so a thread
+// keeps the next group of IPG levels' buoyancies in flight while it integrates the present one. The
+// interface heights are running sums upwards, needed downwards: every IPG-th sum of the block's columns
+// and of the next column and row is kept in shared memory, and a group's heights are summed again from
+// there (the same operations, so the same values) -- all of them in shared memory left room for 20 warps
+// per SM. 1024x1024x40 FP32: 205 -> 125 us.
+constexpr int IPZ_W = 33, IPZ_H = 5, IPG = 4;
+template <class R3>
+__global__ void __launch_bounds__(128) k_ip(Dev d, Bc3<R3> s) {
   chain_sync();
   extern __shared__ unsigned char ip_smem[];
   R3* const zsm = reinterpret_cast<R3*>(ip_smem);
-  auto zsh = [&](int k, int r, int q) -> R3& { return zsm[(k * IPZ_H + r) * IPZ_W + q]; };
+  // the height z(IPG*q) of the block's column (r, c); z(0) = -H
+  auto zck = [&](int q, int r, int c) -> R3& { return zsm[(q * IPZ_H + r) * IPZ_W + c]; };
   const int tx = threadIdx.x, ty = threadIdx.y;
-  if constexpr (ZS) {
+  const int kmax = d.kmax;
+  V3<R3> hn{d, s.f3[HN]};
+  {
     const int i0 = blockIdx.x * 32 + d.imin - HALO, j0 = blockIdx.y * 4 + d.jmin - HALO;
-    V3<R3> hn{d, s.f3[HN]};
     V2 H{d, s.f2[HH]};
     I2 az{d, s.az};
     for (int p = ty * 32 + tx; p < IPZ_W * IPZ_H; p += 128) {
-      const int r = p / IPZ_W, q = p - r * IPZ_W;
-      const int ii = i0 + q, jj = j0 + r;
-      // k_zz at (ii, jj); dry columns and those outside the plane are never read
+      const int r = p / IPZ_W, c = p - r * IPZ_W;
+      const int ii = i0 + c, jj = j0 + r;
+      // dry columns and those outside the plane are never read
       if (ii > d.imax + HALO || jj > d.jmax + HALO || az(ii, jj) < 1) continue;
-      const R3 h = hn(ii, jj, d.kmax);
-      R3 z = R3(-H(ii, jj)) + h;
-      zsh(1, r, q) = z;
-      for (int k = 2; k <= d.kmax; ++k) {
+      const R3 h = hn(ii, jj, kmax);
+      R3 z = R3(-H(ii, jj));
+      zck(0, r, c) = z;
+      for (int k = 1; k <= kmax - 1; ++k) {
         z = z + h;
-        zsh(k, r, q) = z;
+        if (k % IPG == 0) zck(k / IPG, r, c) = z;
       }
     }
-    __syncthreads();
   }
+  __syncthreads();
   GB_IJ_HALO
-  V3<R3> hun{d, s.f3[HUN]}, hvn{d, s.f3[HVN]}, buoy{d, s.f3[BUOY]}, idpdx{d, s.f3[IDPDX]}, idpdy{d, s.f3[IDPDY]},
-      zzg{d, const_cast<R3*>(zzp)};
-  // the interface height at level k of the point (di = dj = 0) or of its neighbour (1, 0) / (0, 1)
-  auto zz = [&](int ii, int jj, int k) -> R3 {
-    if constexpr (ZS) return zsh(k, ty + (jj - j), tx + (ii - i));
-    else return zzg(ii, jj, k);
-  };
+  V3<R3> hun{d, s.f3[HUN]}, hvn{d, s.f3[HVN]}, buoy{d, s.f3[BUOY]}, idpdx{d, s.f3[IDPDX]}, idpdy{d, s.f3[IDPDY]};
   idpdx(i, j, 0) = R3(0);
   idpdy(i, j, 0) = R3(0);
   if (i < d.imin || i > d.imax || j < d.jmin || j > d.jmax) return;
   I2 au{d, s.au}, av{d, s.av};
-  const int kmax = d.kmax;
   const R3 half = R3(0.5);
-  // the point's U and V columns side by side: each a downward integral with its face's layer
-  // height (level-constant with equidistant sigma layers: read once) and its neighbour across the
-  // face ((i+1, j) and (i, j+1)); the loads of B levels of both columns are issued before their
-  // stores, the point's own buoyancy and interface heights loaded once for both
+  // each column a downward integral with its face's layer height (level-constant with equidistant
+  // sigma layers: read once) and its neighbour across the face ((i+1, j) and (i, j+1))
   const bool uc = au(i, j) >= 1, vc = av(i, j) >= 1;
   if (!uc && !vc) return;
   struct Col {
@@ -151,42 +148,60 @@ __global__ void k_ip(Dev d, Bc3<R3> s, const R3* zzp) {
     c.prgr = c.grdl * half * c.hk1;
     out(i, j, kmax) = c.hk1 * c.prgr;
   };
-  auto level = [&](Col& c, V3<R3>& out, int k, R3 b1, R3 b0, R3 z1, R3 z0) {
+  auto level = [&](Col& c, R3 b1, R3 b0, R3 z1, R3 z0) -> R3 {
     const R3 grdu = c.grdl;
     c.grdl = (b1 - b0) * c.dm1;
     const R3 buoyu = c.buoyl;
     c.buoyl = half * (b1 + b0);
     const R3 dz = (z1 - z0) * c.dm1;
     c.prgr = c.prgr + half * (grdu + c.grdl) * half * (c.hc + c.hk1) - dz * (buoyu - c.buoyl);
-    out(i, j, k) = c.hc * c.prgr;
     c.hk1 = c.hc;
+    return c.hc * c.prgr;
   };
   Col cu{}, cv{};
   if (uc) start(cu, hun, idpdx, 1, 0, R3(1.0 / d.dx));
   if (vc) start(cv, hvn, idpdy, 0, 1, R3(1.0 / d.dy));
-  constexpr int B = sizeof(R3) == 4 ? 8 : 4;
-  int k = kmax - 1;
-  for (; k >= B; k -= B) {
-    R3 b0[B], z0[B], bu[B], zu[B], bv[B], zv[B];
+  const R3 h0 = hn(i, j, kmax), hu = hn(i + 1, j, kmax), hv = hn(i, j + 1, kmax);
+  // buoyancies of the levels IPG*q+1 .. IPG*q+IPG of the three columns (levels above kmax-1 and
+  // columns without a face are loaded, in bounds, and not used)
+  const long long sj = d.sj, sk = d.sk, c0 = d.ix(i, j);
+  const R3* const bp = s.f3[BUOY] + c0;
+  R3 *const ox = s.f3[IDPDX] + c0, *const oy = s.f3[IDPDY] + c0;
+  R3 n0[IPG], nu[IPG], nv[IPG];
+  auto load = [&](int q) {
 #pragma unroll
-    for (int m = 0; m < B; ++m) {
-      b0[m] = buoy(i, j, k - m);
-      z0[m] = zz(i, j, k - m);
-      bu[m] = uc ? buoy(i + 1, j, k - m) : R3(0);
-      zu[m] = uc ? zz(i + 1, j, k - m) : R3(0);
-      bv[m] = vc ? buoy(i, j + 1, k - m) : R3(0);
-      zv[m] = vc ? zz(i, j + 1, k - m) : R3(0);
+    for (int m = 0; m < IPG; ++m) {
+      const R3* p = bp + min(IPG * q + 1 + m, kmax - 1) * sk;
+      n0[m] = p[0];
+      nu[m] = p[1];
+      nv[m] = p[sj];
+    }
+  };
+  int q = (kmax - 2 + IPG) / IPG - 1;  // the group of level kmax-1 (-1: kmax = 1)
+  if (q >= 0) load(q);
+  for (; q >= 0; --q) {
+    R3 b0[IPG], bu[IPG], bv[IPG], z0[IPG], zu[IPG], zv[IPG];
+#pragma unroll
+    for (int m = 0; m < IPG; ++m) {
+      b0[m] = n0[m];
+      bu[m] = nu[m];
+      bv[m] = nv[m];
+    }
+    if (q > 0) load(q - 1);
+    R3 a = zck(q, ty, tx), b = zck(q, ty, tx + 1), c = zck(q, ty + 1, tx);
+#pragma unroll
+    for (int m = 0; m < IPG; ++m) {
+      z0[m] = a = a + h0;
+      zu[m] = b = b + hu;
+      zv[m] = c = c + hv;
     }
 #pragma unroll
-    for (int m = 0; m < B; ++m) {
-      if (uc) level(cu, idpdx, k - m, bu[m], b0[m], zu[m], z0[m]);
-      if (vc) level(cv, idpdy, k - m, bv[m], b0[m], zv[m], z0[m]);
+    for (int m = IPG - 1; m >= 0; --m) {
+      const int k = IPG * q + 1 + m;
+      if (k > kmax - 1) continue;
+      if (uc) ox[k * sk] = level(cu, bu[m], b0[m], zu[m], z0[m]);
+      if (vc) oy[k * sk] = level(cv, bv[m], b0[m], zv[m], z0[m]);
     }
-  }
-  for (; k >= 1; --k) {
-    const R3 b0 = buoy(i, j, k), z0 = zz(i, j, k);
-    if (uc) level(cu, idpdx, k, buoy(i + 1, j, k), b0, zz(i + 1, j, k), z0);
-    if (vc) level(cv, idpdy, k, buoy(i, j + 1, k), b0, zz(i, j + 1, k), z0);
   }
 }
 
@@ -1700,16 +1715,15 @@ int run_bc3(int which, const Dev& d, cudaStream_t st, const Bc3<R3>& s, R3* cons
   switch (which) {
     case BC3_BF3D: launch_chained(k_bf3d<R3>, plane_grid(d, blk), blk, 0, st, d, s); break;
     case BC3_ZZ: launch_chained(k_zz<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6]); break;
-    case BC3_IP:
-      if constexpr (sizeof(R3) == 4) {  // the interface heights formed in shared memory (no k_zz)
-        const size_t dyn = (size_t)(d.kmax + 1) * IPZ_H * IPZ_W * sizeof(R3);
-        const cudaError_t e = cudaFuncSetAttribute(k_ip<R3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    case BC3_IP: {
+      const size_t dyn = (size_t)((d.kmax + IPG - 1) / IPG) * IPZ_H * IPZ_W * sizeof(R3);
+      if (dyn > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(k_ip<R3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
         if (e != cudaSuccess) return (int)e;
-        launch_chained(k_ip<R3, true>, plane_grid(d, blk), blk, dyn, st, d, s, nullptr);
-      } else {
-        launch_chained(k_ip<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6]);
       }
+      launch_chained(k_ip<R3>, plane_grid(d, blk), blk, dyn, st, d, s);
       break;
+    }
     case BC3_ZZ_LIN: launch_chained(k_zz_lin<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6]); break;
     case BC3_IP_LIN: launch_chained(k_ip_lin<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6]); break;
     case BC3_IP_SW: launch_chained(k_ip_sw<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6]); break;
