@@ -113,43 +113,70 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
   const int q = threadIdx.x, ty = threadIdx.y;
   const int ii = ii0 - 4 + q;
   const bool iin = ii >= 0 && ii < ni;
-  for (int r = ty; r < RH; r += FTY) {
-    const int jj = jj0 - 2 + r;
-    T f0 = zero, ua = zero, dua = zero, va = zero, dva = zero, dio = zero, oq = zero;
-    uint8_t a = 0, b = 0, c2 = 0, e2 = 0;
-    if (iin && jj >= 0 && jj < nj) {
-      const long long c = (long long)jj * sj + ii;
-      if (bf.r) oq = DIR == 0 ? bf_quot<T>(V[c], DV[c]) : bf_quot<T>(U[c], DU[c]);
-      a = mflux_u[c];
-      b = mflux_v[c];
-      c2 = mupd_u[c];
-      e2 = mupd_v[c];
-      dio = T(DIR == 0 ? DU[c] : DV[c]);
-      const long long cn = DIR == 0 ? c + 1 : c + sj;  // the next U (V) point
-      const bool ok = DIR == 0 ? (ii <= ni - 2) : (jj <= nj - 2);
-      if (ok) {
-        // FP32 working copies: the approximate division (2 ulp); FP64 arrays: the reference's quotient
-        if constexpr (sizeof(T) == 4 && sizeof(TI) == 4)
-          f0 = DIR == 0 ? __fdividef(U[c], DU[c]) : __fdividef(V[c], DV[c]);
-        else
-          f0 = T(DIR == 0 ? U[c] / DU[c] : V[c] / DV[c]);
-        ua = T(0.5 * (U[c] + U[cn]));
-        va = T(0.5 * (V[c] + V[cn]));
-        dua = T(0.5 * (DU[c] + DU[cn]));
-        dva = T(0.5 * (DV[c] + DV[cn]));
+  // SB region rows of a thread at a time, their loads issued together: small tiles (few blocks per SM, a
+  // block's latency is the time) stage every row in one go, large ones (32 registers per thread) one
+  constexpr int SB = RW == 32 ? (RH + FTY - 1) / FTY : 1;
+  for (int rb = ty; rb < RH; rb += SB * FTY) {
+    TI u0[SB], v0[SB], du0[SB], dv0[SB], u1[SB], v1[SB], du1[SB], dv1[SB];
+    uint8_t a[SB], b[SB], c2[SB], e2[SB];
+    bool in[SB], ok[SB];
+#pragma unroll
+    for (int m = 0; m < SB; ++m) {
+      const int r = rb + m * FTY, jj = jj0 - 2 + r;
+      in[m] = r < RH && iin && jj >= 0 && jj < nj;
+      ok[m] = in[m] && (DIR == 0 ? (ii <= ni - 2) : (jj <= nj - 2));  // the next U (V) point exists
+      const long long c = (long long)jj * sj + ii, cn = DIR == 0 ? c + 1 : c + sj;
+      u0[m] = v0[m] = du0[m] = dv0[m] = u1[m] = v1[m] = du1[m] = dv1[m] = TI(0);
+      a[m] = b[m] = c2[m] = e2[m] = 0;
+      if (in[m]) {
+        a[m] = mflux_u[c];
+        b[m] = mflux_v[c];
+        c2[m] = mupd_u[c];
+        e2[m] = mupd_v[c];
+        u0[m] = U[c];
+        v0[m] = V[c];
+        du0[m] = DU[c];
+        dv0[m] = DV[c];
+      }
+      if (ok[m]) {
+        u1[m] = U[cn];
+        v1[m] = V[cn];
+        du1[m] = DU[cn];
+        dv1[m] = DV[cn];
       }
     }
-    sm.F0[r][q] = f0;
-    sm.Q[r][q] = oq;
-    sm.Ua[r][q] = ua;
-    sm.DUa[r][q] = dua;
-    sm.Va[r][q] = va;
-    sm.DVa[r][q] = dva;
-    sm.Di[r][q] = dio;
-    sm.mfu[r][q] = a;
-    sm.mfv[r][q] = b;
-    sm.mpu[r][q] = c2;
-    sm.mpv[r][q] = e2;
+#pragma unroll
+    for (int m = 0; m < SB; ++m) {
+      const int r = rb + m * FTY;
+      if (SB > 1 && r >= RH) break;
+      T f0 = zero, ua = zero, dua = zero, va = zero, dva = zero, dio = zero, oq = zero;
+      if (in[m]) {
+        if (bf.r) oq = DIR == 0 ? bf_quot<T>(v0[m], dv0[m]) : bf_quot<T>(u0[m], du0[m]);
+        dio = T(DIR == 0 ? du0[m] : dv0[m]);
+      }
+      if (ok[m]) {
+        // FP32 working copies: the approximate division (2 ulp); FP64 arrays: the reference's quotient
+        if constexpr (sizeof(T) == 4 && sizeof(TI) == 4)
+          f0 = DIR == 0 ? __fdividef(u0[m], du0[m]) : __fdividef(v0[m], dv0[m]);
+        else
+          f0 = T(DIR == 0 ? u0[m] / du0[m] : v0[m] / dv0[m]);
+        ua = T(0.5 * (u0[m] + u1[m]));
+        va = T(0.5 * (v0[m] + v1[m]));
+        dua = T(0.5 * (du0[m] + du1[m]));
+        dva = T(0.5 * (dv0[m] + dv1[m]));
+      }
+      sm.F0[r][q] = f0;
+      sm.Q[r][q] = oq;
+      sm.Ua[r][q] = ua;
+      sm.DUa[r][q] = dua;
+      sm.Va[r][q] = va;
+      sm.DVa[r][q] = dva;
+      sm.Di[r][q] = dio;
+      sm.mfu[r][q] = a[m];
+      sm.mfv[r][q] = b[m];
+      sm.mpu[r][q] = c2[m];
+      sm.mpv[r][q] = e2[m];
+    }
   }
   __syncthreads();
   // ---- the sweeps. A thread takes region column qc of the rows below; the two warps of a row
@@ -299,14 +326,20 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
   }
 }
 
+// Threads per SM the registers are held to. FP32 working copies in large tiles: 2048 (32 registers, no
+// spills; the shared memory holds them): the issue-bound sweeps then have 64 warps to choose from
+// instead of 48. FP64 arrays: 1024 (2048x2048, 20 micro steps: 20.6 ms; 27.1 at 512). Small tiles: 512, as
+// they run one or two to an SM and 1024 spilled (128x96: 467 against 512 us).
+template <class TI, class TL>
+constexpr int adv2d_threads() { return TL::RW == 32 ? 512 : sizeof(TI) == 4 ? 2048 : 1024; }
+
 // Both components in one launch (blockIdx.z = 0: UEx on the U grid, 1: VEx on the V grid): one grid,
-// one tail. FP32 working copies: 2048 threads per SM (32 registers, no spills; the shared memory holds
-// them): the issue-bound sweeps then have 64 warps to choose from instead of 48. FP64 arrays: 1024.
+// one tail.
 struct Adv2dMasks {
   const uint8_t *mflux_u, *mflux_v, *mupd_u, *mupd_v;
 };
 template <class TL, class T, int S, class TI>
-__global__ void __launch_bounds__(TL::FT, (sizeof(TI) == 4 ? 2048 : 1024) / TL::FT)
+__global__ void __launch_bounds__(TL::FT, adv2d_threads<TI, TL>() / TL::FT)
     k_uvadv2d_both(Dev d, T dt, const TI* __restrict__ U, const TI* __restrict__ V, const TI* __restrict__ DU,
                    const TI* __restrict__ DV, Adv2dMasks mu, Adv2dMasks mv, TI* __restrict__ UEx, TI* __restrict__ VEx,
                    Bf2Args<TI> bfu, Bf2Args<TI> bfv) {

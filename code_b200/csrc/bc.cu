@@ -236,81 +236,70 @@ __global__ void k_finalise2d(Dev d, T dt, T* f, const T* Do, const T* adv, const
 // every interior point and stores it, then updates its own velocity with it -- one launch where
 // the momentum / Coriolis pair took two (the other velocity is not written by this kernel, so no
 // point reads a value another thread changes).
-template <int DIR, bool MIX, bool COR = false>
-__global__ void k_momentum(Dev d, Bc2 s, Bc2W w) {
+// Every input is loaded before the first store and before the mask is looked at: the state's fields may
+// alias as far as the compiler knows, so a load after a store would wait for the store's inputs, and a
+// small domain's time is the number of such waits (with k_sealevel_depth: 128x96, 20 micro steps 566 ->
+// 487 us; 2048x2048 FP64 22.8 -> 21.4 ms with its macro step).
+template <int DIR, bool COR>
+__global__ void k_momentum(Dev d, Bc2 s) {
   chain_sync();
   GB_IJ2
   if (!interior(d, i, j)) return;
+  const long long c = d.ix(i, j), sj = d.sj;
+  const long long n = c + (DIR == 0 ? 1 : sj);  // the next T point along the component
+  const int m = (DIR == 0 ? s.au : s.av)[c];
+  double* const X = s.f2[DIR == 0 ? U_ : V_];
+  double* const fC = s.f2[DIR == 0 ? FV : FU];
+  double o0 = 0.0, o1 = 0.0, o2 = 0.0, o3 = 0.0, cor = 0.0, fCo = 0.0;
   if constexpr (COR) {
-    if (DIR == 0) {  // fV on U points from V
-      auto V = f2a<MIX, V_>(d, s, w);
-      auto fV = f2a<MIX, FV>(d, s, w);
-      W2 coru{d, s.f2[CORU]};
-      M2 au{d, s.au};
-      if (au(i, j) >= 1) {
-        const double Vloc = 0.25 * ((double)V(i, j - 1) + (double)V(i + 1, j - 1) + (double)V(i, j) + (double)V(i + 1, j));
-        fV(i, j) = coru(i, j) * Vloc;
-      } else {
-        fV(i, j) = 0.0;
-      }
-    } else {  // fU on V points from U
-      auto U = f2a<MIX, U_>(d, s, w);
-      auto fU = f2a<MIX, FU>(d, s, w);
-      W2 corv{d, s.f2[CORV]};
-      M2 av{d, s.av};
-      if (av(i, j) >= 1) {
-        const double Uloc = 0.25 * ((double)U(i - 1, j) + (double)U(i, j) + (double)U(i - 1, j + 1) + (double)U(i, j + 1));
-        fU(i, j) = corv(i, j) * Uloc;
-      } else {
-        fU(i, j) = 0.0;
-      }
+    if (DIR == 0) {  // V around the U point
+      const double* V = s.f2[V_];
+      o0 = V[c - sj];
+      o1 = V[c + 1 - sj];
+      o2 = V[c];
+      o3 = V[c + 1];
+      cor = s.f2[CORU][c];
+    } else {  // U around the V point
+      const double* U = s.f2[U_];
+      o0 = U[c - 1];
+      o1 = U[c];
+      o2 = U[c - 1 + sj];
+      o3 = U[c + sj];
+      cor = s.f2[CORV][c];
     }
+  } else {
+    fCo = fC[c];
   }
-  M2 mask{d, DIR == 0 ? s.au : s.av};
-  if (!(mask(i, j) == 1 || mask(i, j) == 2)) return;
-  auto X = f2a<MIX, DIR == 0 ? U_ : V_>(d, s, w);
-  auto DX = f2a<MIX, DIR == 0 ? DU : DV>(d, s, w);
-  auto D = f2a<MIX, D_>(d, s, w);
-  auto airp = f2a<MIX, AIRP>(d, s, w);
-  auto taus = f2a<MIX, DIR == 0 ? TAUSX : TAUSY>(d, s, w);
-  auto Slr_ = f2a<MIX, DIR == 0 ? SLRU : SLRV>(d, s, w);
-  auto dry = f2a<MIX, DIR == 0 ? DRY_U : DRY_V>(d, s, w);
-  auto fC = f2a<MIX, DIR == 0 ? FV : FU>(d, s, w);
-  auto Ex = f2a<MIX, DIR == 0 ? UEX : VEX>(d, s, w);
-  auto Slx = f2a<MIX, DIR == 0 ? SLUX : SLVX>(d, s, w);
-  auto r = f2a<MIX, DIR == 0 ? RU : RV>(d, s, w);
-  W2 z{d, s.f2[Z]}, H{d, s.f2[HH]};
+  const double Xo = X[c], DXo = s.f2[DIR == 0 ? DU : DV][c], dryo = s.f2[DIR == 0 ? DRY_U : DRY_V][c],
+               Exo = s.f2[DIR == 0 ? UEX : VEX][c], Slxo = s.f2[DIR == 0 ? SLUX : SLVX][c],
+               Slro = s.f2[DIR == 0 ? SLRU : SLRV][c], ro = s.f2[DIR == 0 ? RU : RV][c];
+  const double *z = s.f2[Z], *H = s.f2[HH], *D = s.f2[D_], *airp = s.f2[AIRP], *taus = s.f2[DIR == 0 ? TAUSX : TAUSY];
+  const double zc = z[c], zn = z[n], Hc = H[c], Hn = H[n], Dc = D[c], Dn = D[n], ac = airp[c], an = airp[n], tc = taus[c],
+               tn = taus[n];
+  if constexpr (COR) {
+    fCo = m >= 1 ? cor * (0.25 * (o0 + o1 + o2 + o3)) : 0.0;
+    fC[c] = fCo;
+  }
+  if (!(m == 1 || m == 2)) return;
   const double g = s.par[P_G], rho_0 = s.par[P_RHO_0], dtm = s.par[P_DTM], min_depth = s.par[P_MIN_DEPTH];
   const double gamma = rho_0 * g;
   const double gammai = 1.0 / gamma;
-  const int di = DIR == 0 ? 1 : 0, dj = DIR == 0 ? 0 : 1;
-  const double zp = fmax(z(i + di, j + dj), -H(i, j) + fmin(min_depth, (double)D(i + di, j + dj)));
-  const double zm = fmax(z(i, j), -H(i + di, j + dj) + fmin(min_depth, (double)D(i, j)));
-  const double zx = (zp - zm + ((double)airp(i + di, j + dj) - (double)airp(i, j)) * gammai) / (DIR == 0 ? d.dx : d.dy);
-  const double tau = 0.5 * ((double)taus(i, j) + (double)taus(i + di, j + dj));
-  const double Slr = X(i, j) > 0.0 ? fmax((double)Slr_(i, j), 0.0) : fmin((double)Slr_(i, j), 0.0);
-  const double Xo = X(i, j), DXo = DX(i, j), dryo = dry(i, j), fCo = fC(i, j), Exo = Ex(i, j), Slxo = Slx(i, j),
-               ro = r(i, j);
+  const double zp = fmax(zn, -Hc + fmin(min_depth, Dn));
+  const double zm = fmax(zc, -Hn + fmin(min_depth, Dc));
+  const double zx = (zp - zm + (an - ac) * gammai) / (DIR == 0 ? d.dx : d.dy);
+  const double tau = 0.5 * (tc + tn);
+  const double Slr = Xo > 0.0 ? fmax(Slro, 0.0) : fmin(Slro, 0.0);
   if (DIR == 0)
-    X(i, j) = (Xo - dtm * (g * DXo * zx + dryo * (-tau / rho_0 - fCo + Exo + Slxo + Slr))) / (1.0 + dtm * ro / DXo);
+    X[c] = (Xo - dtm * (g * DXo * zx + dryo * (-tau / rho_0 - fCo + Exo + Slxo + Slr))) / (1.0 + dtm * ro / DXo);
   else
-    X(i, j) = (Xo - dtm * (g * DXo * zx + dryo * (-tau / rho_0 + fCo + Exo + Slxo + Slr))) / (1.0 + dtm * ro / DXo);
+    X[c] = (Xo - dtm * (g * DXo * zx + dryo * (-tau / rho_0 + fCo + Exo + Slxo + Slr))) / (1.0 + dtm * ro / DXo);
 }
 
 // The mixed micro step's form of k_momentum: the same update with the elevation gradient's
 // difference zp - zm taken in FP64 (the elevations are FP64) and every other operation in FP32 on
-// the FP32 working copies (the Coriolis term with COR as well). Split into the Coriolis term and
-// the update of one point (momentum_core_f32 from the point's inputs), which the one- and
-// two-point kernels share.
+// the FP32 working copies (the Coriolis term with COR as well). The update of one point from its
+// inputs (momentum_core_f32) is shared by the one- and the two-point kernel.
 //
-// The Coriolis term of the DIR update at c (DIR 0: fV on U points from V at c-sj, c+1-sj, c, c+1;
-// DIR 1: fU on V points from U at c-1, c, c-1+sj, c+sj), given those four values in that order.
-template <int DIR>
-__device__ __forceinline__ float cor_term_f32(const Bc2& s, const Bc2W& w, long long c, float a, float b, float e,
-                                              float f) {
-  const int m = DIR == 0 ? w.m8[1][c] : w.m8[2][c];
-  return m >= 1 ? float(s.f2[DIR == 0 ? CORU : CORV][c]) * (0.25f * (a + b + e + f)) : 0.f;
-}
 // The new velocity of the DIR update at one point from its inputs: old value Xo, Coriolis term fCo,
 // elevation, depth H, total depth D, air pressure and surface stress at the point (c) and at the
 // next T point along the component (n), then the point's slow term, face depth, drying factor,
@@ -331,43 +320,50 @@ __device__ __forceinline__ float momentum_core_f32(const Dev& d, const Bc2& s, f
   const float fc = DIR == 0 ? -fCo : fCo;
   return (Xo - dtm * (g * DXo * zx + dryo * (-tau / rho_0 + fc + Exo + Slxo + Slr))) / (1.f + dtm * ro / DXo);
 }
-// The new velocity of the DIR update at an interior point c whose mask is 1 or 2, from its old value
-// Xo and the Coriolis term fCo.
-template <int DIR>
-__device__ __forceinline__ float momentum_new_f32(const Dev& d, const Bc2& s, const Bc2W& w, long long c, float Xo,
-                                                  float fCo) {
-  const long long dn = DIR == 0 ? 1 : d.sj;  // the next T point along the component
-  const float* D = w.w[D_];
-  const float* airp = w.w[AIRP];
-  const float* taus = w.w[DIR == 0 ? TAUSX : TAUSY];
-  const double* z = s.f2[Z];
-  const float* H = w.w[HH];
-  return momentum_core_f32<DIR>(d, s, Xo, fCo, z[c], z[c + dn], H[c], H[c + dn], D[c], D[c + dn], airp[c],
-                                airp[c + dn], taus[c], taus[c + dn], w.w[DIR == 0 ? SLRU : SLRV][c],
-                                w.w[DIR == 0 ? DU : DV][c], w.w[DIR == 0 ? DRY_U : DRY_V][c],
-                                w.w[DIR == 0 ? UEX : VEX][c], w.w[DIR == 0 ? SLUX : SLVX][c],
-                                w.w[DIR == 0 ? RU : RV][c]);
-}
-
+// Loads first, as in k_momentum.
 template <int DIR, bool COR>
 __global__ void k_momentum_f32(Dev d, Bc2 s, Bc2W w) {
   chain_sync();
   GB_IJ2
   if (!interior(d, i, j)) return;
-  const long long c = d.ix(i, j);
+  const long long c = d.ix(i, j), sj = d.sj;
+  const long long n = c + (DIR == 0 ? 1 : sj);  // the next T point along the component
+  const int m = DIR == 0 ? w.m8[1][c] : w.m8[2][c];
+  float* const X = w.w[DIR == 0 ? U_ : V_];
+  float* const fC = w.w[DIR == 0 ? FV : FU];
+  float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f, fCo = 0.f;
+  double cor = 0.0;
   if constexpr (COR) {
     if (DIR == 0) {  // fV on U points from V
       const float* V = w.w[V_];
-      w.w[FV][c] = cor_term_f32<0>(s, w, c, V[c - d.sj], V[c + 1 - d.sj], V[c], V[c + 1]);
+      o0 = V[c - sj];
+      o1 = V[c + 1 - sj];
+      o2 = V[c];
+      o3 = V[c + 1];
+      cor = s.f2[CORU][c];
     } else {  // fU on V points from U
       const float* U = w.w[U_];
-      w.w[FU][c] = cor_term_f32<1>(s, w, c, U[c - 1], U[c], U[c - 1 + d.sj], U[c + d.sj]);
+      o0 = U[c - 1];
+      o1 = U[c];
+      o2 = U[c - 1 + sj];
+      o3 = U[c + sj];
+      cor = s.f2[CORV][c];
     }
+  } else {
+    fCo = fC[c];
   }
-  const int m = DIR == 0 ? w.m8[1][c] : w.m8[2][c];
+  const float *D = w.w[D_], *airp = w.w[AIRP], *taus = w.w[DIR == 0 ? TAUSX : TAUSY], *H = w.w[HH];
+  const double zc = s.f2[Z][c], zn = s.f2[Z][n];
+  const float Xo = X[c], Hc = H[c], Hn = H[n], Dc = D[c], Dn = D[n], ac = airp[c], an = airp[n], tc = taus[c], tn = taus[n],
+              sl = w.w[DIR == 0 ? SLRU : SLRV][c], DX = w.w[DIR == 0 ? DU : DV][c],
+              dry = w.w[DIR == 0 ? DRY_U : DRY_V][c], Ex = w.w[DIR == 0 ? UEX : VEX][c],
+              Slx = w.w[DIR == 0 ? SLUX : SLVX][c], ro = w.w[DIR == 0 ? RU : RV][c];
+  if constexpr (COR) {
+    fCo = m >= 1 ? float(cor) * (0.25f * (o0 + o1 + o2 + o3)) : 0.f;
+    fC[c] = fCo;
+  }
   if (!(m == 1 || m == 2)) return;
-  float* X = w.w[DIR == 0 ? U_ : V_];
-  X[c] = momentum_new_f32<DIR>(d, s, w, c, X[c], w.w[DIR == 0 ? FV : FU][c]);
+  X[c] = momentum_core_f32<DIR>(d, s, Xo, fCo, zc, zn, Hc, Hn, Dc, Dn, ac, an, tc, tn, sl, DX, dry, Ex, Slx, ro);
 }
 
 // k_momentum_f32 on two neighbouring points per thread (region columns 2t and 2t+1 of a row, for
@@ -569,63 +565,71 @@ __global__ void k_depth_update(Dev d, Bc2 s, Bc2W w) {
 // update_2d_bdy has set their elevations in z). The elevations ping-pong between the state's z and
 // zo arrays: s.f2[Z] holds the elevations before the step and is only read; the new ones go to
 // s.f2[ZO], so the old array is exactly the reference's zo = z of sealevel.F90:89 and the caller
-// swaps the two pointers after the launch. The depths of a U (V) point need the new elevation of the next T point, which the
-// thread forms itself from the same inputs with the same expression (no thread reads a value
+// swaps the two pointers after the launch. The depths of a U (V) point need the new elevation of the
+// next T point, which the thread forms itself from the same inputs with the same expression (no thread reads a value
 // that another writes). Same values as the two kernels, bit for bit. flags: bit 0 accumulates
 // Uint/Vint; bit 1 writes the drying factor dry_z, which no micro-step kernel reads: the caller asks
 // for it on the micro steps whose state a macro step or the host reads next.
+// Loads first, as in k_momentum (the addresses of neighbours outside the plane are the point's own).
 template <bool MIX>
 __global__ void k_sealevel_depth(Dev d, Bc2 s, Bc2W w, int flags) {
   chain_sync();
-  const int accumulate = flags & 1;
   GB_IJ2
-  auto U = f2a<MIX, U_>(d, s, w);
-  auto V = f2a<MIX, V_>(d, s, w);
-  auto D = f2a<MIX, D_>(d, s, w);
-  auto DU_ = f2a<MIX, DU>(d, s, w);
-  auto DV_ = f2a<MIX, DV>(d, s, w);
-  auto dry_u = f2a<MIX, DRY_U>(d, s, w);
-  auto dry_v = f2a<MIX, DRY_V>(d, s, w);
-  auto fwf = f2a<MIX, FWF>(d, s, w);
-  auto H = f2a<MIX, HH>(d, s, w);
-  auto HU_ = f2a<MIX, HU>(d, s, w);
-  auto HV_ = f2a<MIX, HV>(d, s, w);
-  W2 zold{d, s.f2[Z]}, znew{d, s.f2[ZO]}, Uint{d, s.f2[UINT]}, Vint{d, s.f2[VINT]}, dry_z{d, s.f2[DRY_Z]};
-  auto az = m2a<MIX>(d, s, w, 0);
-  auto au = m2a<MIX>(d, s, w, 1);
-  auto av = m2a<MIX>(d, s, w, 2);
-  const double dtm = s.par[P_DTM];
-  // sealevel.F90:94-108 at (ii, jj)
-  auto zn = [&](int ii, int jj) -> double {
-    const double zo_ = zold(ii, jj);
-    if (interior(d, ii, jj) && az(ii, jj) == 1)
-      return zo_ - dtm * (((double)U(ii, jj) * d.dy - (double)U(ii - 1, jj) * d.dy) +
-                          ((double)V(ii, jj) * d.dx - (double)V(ii, jj - 1) * d.dx)) * d.ard1 +
-             dtm * fwf(ii, jj);
-    return zo_;
+  using E = std::conditional_t<MIX, float, double>;  // the type of the working fields
+  auto fld = [&](int q) -> E* {
+    if constexpr (MIX) return w.w[q];
+    else return s.f2[q];
   };
-  if (accumulate) {
-    Uint(i, j) = Uint(i, j) + U(i, j);
-    Vint(i, j) = Vint(i, j) + V(i, j);
+  auto msk = [&](int q, long long c) -> int {
+    if constexpr (MIX) return w.m8[q][c];
+    else return (q == 0 ? s.az : q == 1 ? s.au : s.av)[c];
+  };
+  const bool east = i < d.imax + HALO, north = j < d.jmax + HALO;
+  const long long c = d.ix(i, j), ce = east ? c + 1 : c, cn = north ? c + d.sj : c;
+  const long long west = i > d.imin - HALO ? 1 : 0, south = j > d.jmin - HALO ? d.sj : 0;
+  const E *U = fld(U_), *V = fld(V_), *fwf = fld(FWF);
+  const double* z = s.f2[Z];
+  const bool acc = flags & 1;
+  const double zc = z[c], ze = z[ce], zN = z[cn];
+  const E u0 = U[c], uw = U[c - west], ue = U[ce], un = U[cn], unw = U[cn - west];
+  const E v0 = V[c], vs = V[c - south], ve = V[ce], ves = V[ce - south], vn = V[cn];
+  const E f0 = fwf[c], fe = fwf[ce], fn = fwf[cn];
+  const E Hc = fld(HH)[c], HUc = fld(HU)[c], HVc = fld(HV)[c];
+  const int a0 = msk(0, c), ae = msk(0, ce), an = msk(0, cn), mu = msk(1, c), mv = msk(2, c);
+  const double ui = acc ? s.f2[UINT][c] : 0.0, vi = acc ? s.f2[VINT][c] : 0.0;
+  E DUn = east ? E(0) : fld(DU)[c], DVn = north ? E(0) : fld(DV)[c];  // not renewed in the last column (row)
+  const double dtm = s.par[P_DTM];
+  // sealevel.F90:94-108 at a point from its inputs
+  auto zn_of = [&](bool upd, double zo, E a, E aw, E b, E bs, E f) -> double {
+    return upd ? zo - dtm * (((double)a * d.dy - (double)aw * d.dy) + ((double)b * d.dx - (double)bs * d.dx)) * d.ard1 +
+                     dtm * f
+               : zo;
+  };
+  const double z0 = zn_of(interior(d, i, j) && a0 == 1, zc, u0, uw, v0, vs, f0);
+  const double z1 = zn_of(interior(d, i + 1, j) && ae == 1, ze, ue, u0, ve, ves, fe);
+  const double z2 = zn_of(interior(d, i, j + 1) && an == 1, zN, un, unw, vn, v0, fn);
+  if (acc) {
+    s.f2[UINT][c] = ui + u0;
+    s.f2[VINT][c] = vi + v0;
   }
-  const double z0 = zn(i, j);
-  znew(i, j) = z0;
+  s.f2[ZO][c] = z0;
   // depth_update.F90:55-110
   const double min_depth = s.par[P_MIN_DEPTH], crit_depth = s.par[P_CRIT_DEPTH];
-  D(i, j) = z0 + H(i, j);
-  if (i <= d.imax + HALO - 1) {
-    const double x = fmax(0.25 * (zold(i, j) + zold(i + 1, j) + z0 + zn(i + 1, j)), -HU_(i, j) + min_depth);
-    DU_(i, j) = x + HU_(i, j);
+  const E Dn = z0 + Hc;
+  fld(D_)[c] = Dn;
+  if (east) {
+    DUn = fmax(0.25 * (zc + ze + z0 + z1), -HUc + min_depth) + HUc;
+    fld(DU)[c] = DUn;
   }
-  if (j <= d.jmax + HALO - 1) {
-    const double x = fmax(0.25 * (zold(i, j) + zold(i, j + 1) + z0 + zn(i, j + 1)), -HV_(i, j) + min_depth);
-    DV_(i, j) = x + HV_(i, j);
+  if (north) {
+    DVn = fmax(0.25 * (zc + zN + z0 + z2), -HVc + min_depth) + HVc;
+    fld(DV)[c] = DVn;
   }
   const double d1 = 2 * min_depth;
   const double d2i = 1.0 / (crit_depth - 2 * min_depth);
-  if ((flags & 2) && az(i, j) > 0) dry_z(i, j) = fmax(0.0, fmin(1.0, (D(i, j) - 0.5 * d1) * d2i));
-  if (au(i, j) > 0) dry_u(i, j) = fmax(0.0, fmin(1.0, (DU_(i, j) - d1) * d2i));
-  if (av(i, j) > 0) dry_v(i, j) = fmax(0.0, fmin(1.0, (DV_(i, j) - d1) * d2i));
+  if ((flags & 2) && a0 > 0) s.f2[DRY_Z][c] = fmax(0.0, fmin(1.0, (Dn - 0.5 * d1) * d2i));
+  if (mu > 0) fld(DRY_U)[c] = fmax(0.0, fmin(1.0, (DUn - d1) * d2i));
+  if (mv > 0) fld(DRY_V)[c] = fmax(0.0, fmin(1.0, (DVn - d1) * d2i));
 }
 
 // k_sealevel_depth<true> on two neighbouring points per thread (region columns 2t and 2t+1 of a row,
@@ -1407,8 +1411,8 @@ int momentum_2d(getm_ctx* ctx, const getm_bc_state* st, const Bc2W* wp, bool cor
   {
     TimerScope ts(ctx, GETM_TIM_BC2D);
     int e;
-    if (!wp && fused && cor) e = launch_chained(k_momentum<DIR, false, true>, grid2(d), kBlk2, 0, cs, d, s, w);
-    else if (!wp) e = launch_chained(k_momentum<DIR, false, false>, grid2(d), kBlk2, 0, cs, d, s, w);
+    if (!wp && fused && cor) e = launch_chained(k_momentum<DIR, true>, grid2(d), kBlk2, 0, cs, d, s);
+    else if (!wp) e = launch_chained(k_momentum<DIR, false>, grid2(d), kBlk2, 0, cs, d, s);
     else if (pairs_ok(d, s, w)) {
       const dim3 gp((d.ni() / 2 + 31) / 32, (d.nj() + 3) / 4, 1);
       if (cor) e = launch_chained(k_momentum_f32v<DIR, true>, gp, kBlk2, 0, cs, d, s, w);
