@@ -21,16 +21,19 @@ namespace gb {
 // launches of fewer large tiles than this take the small ones (two large tiles per SM)
 constexpr long long TILE2D_SMALL = 296;
 // A block of RW x FTY threads (lane x <-> region column) owns FX x FY cells of a staged region of
-// RW x RH, i in [-4, FX+3], j in [-2, FY+1]. Two sizes: 56 x 16 own cells (64 x 8 threads) where the
-// domain gives every SM work, 24 x 8 (32 x 4 threads, 1.7 times the halo) below, where the time is
-// the latency of one block: 128 x 96 FP64, both components 26 us in two launches of 21 large tiles,
-// 10 us in one launch of 156 small ones.
-template <int RW_, int FTY_>
+// RW x RH, i in [-4, FX+3], j in [-2, FY+1]. Two sizes: 56 x 16 own cells (64 x 8 threads, two own
+// rows each) where the domain gives every SM work, and 24 x 8 (32 x 8 threads, one own row each)
+// below, where the time is the latency of one block: a thread's chain of divisions and logarithms
+// then runs once instead of twice, for 1.9 times the halo work on SMs that would idle. Whole step with one
+// and two own rows per thread: 128 x 96 FP64 379 against 464 us, 80 x 96 x 12 FP64 563 against 640,
+// 259 x 251 x 17 mixed 671 against 682, 300 x 300 x 12 FP64 1204 against 1242, mixed 720 against 708.
+template <int RW_, int FTY_, int RPT_>
 struct Tile2d {
-  static constexpr int RW = RW_, FTY = FTY_, FX = RW - 8, FY = 2 * FTY, RH = FY + 4, FT = RW * FTY;
+  static constexpr int RW = RW_, FTY = FTY_, RPT = RPT_;  // RPT: own rows per thread
+  static constexpr int FX = RW - 8, FY = RPT * FTY, RH = FY + 4, FT = RW * FTY;
 };
-using TileLarge = Tile2d<64, 8>;
-using TileSmall = Tile2d<32, 4>;
+using TileLarge = Tile2d<64, 8, 2>;
+using TileSmall = Tile2d<32, 8, 1>;
 
 // k*(a*s - b*s)*c as single rounded operations in this order: the volume and flux differences of
 // the cell updates. FP64: the plain operations (the FP64 build contracts nothing); FP32: explicit
@@ -100,7 +103,7 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
                                              const uint8_t* __restrict__ mflux_v,
                                              const uint8_t* __restrict__ mupd_u, const uint8_t* __restrict__ mupd_v,
                                              TI* __restrict__ Ex, const Bf2Args<TI>& bf) {
-  constexpr int FX = TL::FX, FY = TL::FY, RW = TL::RW, RH = TL::RH, FTY = TL::FTY;
+  constexpr int FX = TL::FX, FY = TL::FY, RW = TL::RW, RH = TL::RH, FTY = TL::FTY, RPT = TL::RPT;
   extern __shared__ unsigned char smem_raw[];
   Adv2dSmem<T, TL>& sm = *reinterpret_cast<Adv2dSmem<T, TL>*>(smem_raw);
   const int ni = d.ni(), nj = d.nj();
@@ -183,13 +186,13 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
   // overlap by one column (warp 0: qc = 0..31, warp 1: qc = 31..62; warp 1's copy of column 31,
   // `dup`, updates and stores nothing), so that the left face flux of every cell a u sweep updates
   // is the flux of the lane before it (a warp shuffle, no shared-memory round trip or barrier).
-  // The own rows of a thread, r = 2 + ty + FTY*m (m = 0, 1), are the same in all three sweeps: their
+  // The own rows of a thread, r = 2 + ty + FTY*m (m < RPT), are the same in all three sweeps: their
   // depths and flux-divergence sums stay in registers.
   const int qc = q - (q >> 5);
   const bool dup = q == 32;
   const int iic = ii0 - 4 + qc;
   const bool qown = qc >= 4 && qc < FX + 4 && !dup;  // own cells q in [4, FX+4)
-  T di[2], acc[2] = {zero, zero};
+  T di[RPT], acc[RPT] = {};
   // ---- sweep 1: u/2 on rows r in [0, RH), cells q in [2, RW-2), faces q in [1, RW-3]
   {
     const T dti = half * dt, cdx = dti / dxu;
@@ -197,10 +200,10 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
     const bool cok = iic >= 1 + sub && iic <= ni - 2 - sub;
     const bool upd = qc >= 2 && qc < RW - 2 && !dup;
 #pragma unroll
-    for (int m = 0; m < 3; ++m) {
+    for (int m = 0; m <= RPT; ++m) {
       // the own rows, then the halo rows 0, 1, RH-2, RH-1 (thread rows 0..3)
-      const int r = m < 2 ? 2 + ty + FTY * m : (ty < 2 ? ty : RH - 4 + ty);
-      if (m == 2 && ty >= 4) continue;
+      const int r = m < RPT ? 2 + ty + FTY * m : (ty < 2 ? ty : RH - 4 + ty);
+      if (m == RPT && ty >= 4) continue;
       T fl = zero;
       if (fok)
         fl = face_flux_s<T, S>(sm.Ua[r][qc], sm.DUa[r][qc], sm.F0[r][qc - 1], sm.F0[r][qc], sm.F0[r][qc + 1],
@@ -217,9 +220,9 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
           const T advn = diff_scaled<T>(half, fl, flm, dyu, ard1);
           fnew = fv_update<T>(Dio, dD, Dn, fio, dt, advn);
           Dio = Dn;
-          if (m < 2 && qown) acc[m] = add_r<T>(acc[m], advn);
+          if (m < RPT && qown) acc[m] = add_r<T>(acc[m], advn);
         }
-        if (m < 2) di[m] = Dio;
+        if (m < RPT) di[m] = Dio;
         sm.F1[r][qc] = fnew;
       }
     }
@@ -242,7 +245,7 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
     __syncthreads();
     if (col) {
 #pragma unroll
-      for (int m = 0; m < 2; ++m) {
+      for (int m = 0; m < RPT; ++m) {
         const int r = 2 + ty + FTY * m;
         const int jj = jj0 - 2 + r;
         const T fio = sm.F1[r][qc];
@@ -265,7 +268,7 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
     const T dti = half * dt, cdx = dti / dxu;
     const bool fok = qc >= 3 && qc <= RW - 5 && iic >= sub && iic <= ni - 2 - sub;
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
+    for (int m = 0; m < RPT; ++m) {
       const int r = 2 + ty + FTY * m;
       T fl = zero;
       if (fok)
@@ -287,7 +290,7 @@ __device__ __forceinline__ void uvadv2d_tile(const Dev& d, T dt, const TI* __res
   // ---- the bottom friction of the own points (bottom_friction.F90:48-150)
   if (bf.r && qown) {
 #pragma unroll
-    for (int m = 0; m < 2; ++m) {
+    for (int m = 0; m < RPT; ++m) {
       const int r = 2 + ty + FTY * m;
       const int jj = jj0 - 2 + r;
       if (iic >= ni || jj >= nj) continue;
