@@ -105,7 +105,7 @@ int step_record(getm_ctx* ctx, R dt, R* f, const R* uu, const R* vv, const R* ww
   // the diffusion's result also goes to sn when the caller keeps the step outputs (only the solved
   // columns are written there -- the only ones the adjoint diffusion reads)
   GB_TIMED(GETM_TIM_ADJ_RECORD, run_vdiff<R>(d, s, dt, cnpar, avmol, f, hn, nuh, ctx->zmask, nullptr, (R*)ctx->scr[0],
-                                             (R*)ctx->scr[1], nullptr, sn), "vdiff");
+                                             nullptr, sn), "vdiff");
   return GETM_OK;
 }
 
@@ -140,7 +140,7 @@ int step_adjoint(getm_ctx* ctx, R dt, R* fbar, R* nubar, const R* uu, const R* v
   const R* Sout = Sn_in;
   if (!Sout) {
     GB_TIMED(GETM_TIM_ADJ, cudaMemcpyAsync(Sn, g, (size_t)n3 * sizeof(R), cudaMemcpyDeviceToDevice, s), "copy g");
-    GB_TIMED(GETM_TIM_ADJ, run_vdiff<R>(d, s, dt, cnpar, avmol, Sn, hn, nuh, ctx->zmask, nullptr, RU, QU), "vdiff");
+    GB_TIMED(GETM_TIM_ADJ, run_vdiff<R>(d, s, dt, cnpar, avmol, Sn, hn, nuh, ctx->zmask, nullptr, RU), "vdiff");
     Sout = Sn;
   }
   GB_TIMED(GETM_TIM_ADJ, run_adj_vdiff<R>(d, s, dt, cnpar, avmol, fbar, tmp, nubar, g, Sout, hn, nuh, ctx->zmask,

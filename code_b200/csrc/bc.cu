@@ -1752,8 +1752,8 @@ int integrate_3d(getm_ctx* ctx, getm_bc_state* st, int n) {
       R3* b3 = (R3*)ctx->bc_scr3;
       GB_TIMED(GETM_TIM_VDIFF,
                run_vdiff2<R3>(d, s, dt, R3(st->par[P_CNPAR]), CH(COL_HN), f3[NUH], st->az, f3[TT],
-                              R3(st->par[P_AVMOLT]), (const R3*)tsrc, b3 + 2 * n3, nullptr, tlo, f3[SS],
-                              R3(st->par[P_AVMOLS]), b3, nullptr, slo, true),
+                              R3(st->par[P_AVMOLT]), (const R3*)tsrc, b3 + 2 * n3, tlo, f3[SS],
+                              R3(st->par[P_AVMOLS]), b3, slo, true),
                "vdiff T, S");
     }
     if (!pair && ip[I_CALC_TEMP]) {
@@ -1763,7 +1763,7 @@ int integrate_3d(getm_ctx* ctx, getm_bc_state* st, int n) {
         return rc;
       if (radn && (rc = temp_sources(nullptr))) return rc;
       GB_TIMED(GETM_TIM_VDIFF, run_vdiff<R3>(d, s, dt, R3(st->par[P_CNPAR]), R3(st->par[P_AVMOLT]), f3[TT], f3[HN],
-                                             f3[NUH], st->az, (const R3*)tsrc, (R3*)ctx->scr[0], (R3*)ctx->scr[1],
+                                             f3[NUH], st->az, (const R3*)tsrc, (R3*)ctx->scr[0],
                                              nullptr, nullptr, tlo),
                "vdiff T");
     }
@@ -1773,7 +1773,7 @@ int integrate_3d(getm_ctx* ctx, getm_bc_state* st, int n) {
                              nullptr, nullptr, ip[I_ADV_VER_ITERS], true, slo)))
         return rc;
       GB_TIMED(GETM_TIM_VDIFF, run_vdiff<R3>(d, s, dt, R3(st->par[P_CNPAR]), R3(st->par[P_AVMOLS]), f3[SS], f3[HN],
-                                             f3[NUH], st->az, (const R3*)nullptr, (R3*)ctx->scr[0], (R3*)ctx->scr[1],
+                                             f3[NUH], st->az, (const R3*)nullptr, (R3*)ctx->scr[0],
                                              nullptr, nullptr, slo),
                "vdiff S");
     }

@@ -411,7 +411,7 @@ static int vdiff_api(getm_ctx* ctx, R dt, R cnpar, R avmol, R* S, const R* hn, c
   int rc = ensure_scratch(ctx, (size_t)n3d(ctx->dev) * sizeof(R));
   if (rc) return rc;
   GB_TIMED(GETM_TIM_VDIFF,
-           run_vdiff<R>(ctx->dev, ctx->stream, dt, cnpar, avmol, S, hn, nuh, az, src, (R*)ctx->scr[0], (R*)ctx->scr[1]),
+           run_vdiff<R>(ctx->dev, ctx->stream, dt, cnpar, avmol, S, hn, nuh, az, src, (R*)ctx->scr[0]),
            "tracer_vdiff");
   return GETM_OK;
 }
@@ -538,7 +538,7 @@ int getm_ctx_destroy(getm_ctx* ctx) {
   cudaFree(ctx->red);
   cudaFree(ctx->cnt);
   cudaFree(ctx->stage);
-  for (auto p : ctx->scr) cudaFree(p);
+  cudaFree(ctx->scr[0]);
   cudaFree(ctx->bc_scr3);
   cudaFree(ctx->bc_scr2);
   cudaFree(ctx->colh);

@@ -130,18 +130,20 @@ static inline int cuda_fail(getm_ctx* c, int e, const char* where) {
     if (_e != 0) return cuda_fail(ctx, _e, where);            \
   } while (0)
 
+// The three 3D scratch arrays, of `bytes` each (rounded up to 256) in one allocation: scr[0] and scr[1] together
+// also hold one array of twice the elements (the diffusion's coefficient pairs).
 static inline int ensure_scratch(getm_ctx* ctx, size_t bytes) {
   if (ctx->scr_bytes >= bytes) return GETM_OK;
-  for (auto& p : ctx->scr) {
-    if (p) cudaFree(p);
-    p = nullptr;
-  }
+  cudaFree(ctx->scr[0]);
+  for (auto& p : ctx->scr) p = nullptr;
   ctx->scr_bytes = 0;
-  for (auto& p : ctx->scr)
-    if (cudaMalloc(&p, bytes) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(ctx, GETM_ERR_NOMEM, "scratch allocation failed");
-    }
+  const size_t pitch = (bytes + 255) / 256 * 256;
+  char* base = nullptr;
+  if (cudaMalloc(&base, 3 * pitch) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(ctx, GETM_ERR_NOMEM, "scratch allocation failed");
+  }
+  for (int q = 0; q < 3; ++q) ctx->scr[q] = base + q * pitch;
   ctx->scr_bytes = bytes;
   return GETM_OK;
 }

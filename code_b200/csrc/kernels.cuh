@@ -932,14 +932,13 @@ __global__ void __launch_bounds__(64) k_sweep_w_iter(Dev d, R dt, R splitfac, in
 // ---------------------------------------------------------------------------------------------
 // One tracer of the implicit vertical diffusion: the old values are read from Sin and the new ones
 // written to S (they may alias) and, when S2 is given, to S2 as well; src (may be null): the
-// temperature form's sources; RU, QU: two scratch 3D arrays; lo: the compensated storage (FP32).
+// temperature form's sources; RQ: scratch of two 3D arrays' size; lo: the compensated storage (FP32).
 template <class R>
 struct VdField {
   const R* Sin;
   R* S;
   const R* src;
-  R* RU;
-  R* QU;
+  R* RQ;
   R* S2;
   __half* lo;
   R avmol;
@@ -952,12 +951,13 @@ struct VdSet {
 // Implicit vertical diffusion (salinity.F90:348-389; temperature form with src) of NF = 1 or 2
 // tracers (do_temperature and do_salinity share hn and nuh). One thread per interior column; the
 // matrix rows are built top-down as the elimination proceeds, ru(k+1)/qu(k+1) carried in registers
-// and ru(k)/qu(k) stored in two scratch 3D arrays per tracer (full occupancy, no shared memory for
-// them: holding them in shared memory measured 1.6x slower at kmax = 50, from the lower occupancy)
-// for the back substitution. With two tracers the thread runs their two eliminations side by side
+// and (ru(k), qu(k)) stored as a pair in a scratch array per tracer (full occupancy, no shared memory
+// for them: holding them in shared memory measured 1.6x slower at kmax = 50, from the lower occupancy;
+// in two arrays, the mixed 2048 x 2048 x 50 launch for two tracers took 2.45 against 2.11 ms, one
+// tracer of 1024 x 1024 x 40 FP64 396 against 348 us) for the back substitution. With two tracers the thread runs their two eliminations side by side
 // (independent chains) and loads hn and nuh once.
 // hsk: the level stride of hn (d.sk; 0 when hn is a 2D array of column heights)
-template <class R, int NF, bool IL = false>
+template <class R, int NF>
 __global__ void __launch_bounds__(128) k_vdiff(Dev d, R dt, R cnpar, VdSet<R, NF> F, const R* __restrict__ hn,
                                                const R* __restrict__ nuh, const int32_t* __restrict__ az,
                                                long long hsk) {
@@ -969,29 +969,18 @@ __global__ void __launch_bounds__(128) k_vdiff(Dev d, R dt, R cnpar, VdSet<R, NF
   const long long c = d.ix(i, j);
   if (az[c] != 1 || kmax <= 1) return;
   const long long sk = d.sk;
-  // the elimination coefficients ru(k), qu(k) of a tracer: two scratch arrays, or (IL) one array of
-  // (ru, qu) pairs at RU (twice the elements), one 8- or 16-byte access per level
+  // the elimination coefficients ru(k), qu(k) of a tracer as pairs: one access per level
   using R2 = std::conditional_t<sizeof(R) == 4, float2, double2>;
   auto put_rq = [&](const VdField<R>& f, int k, R r, R q) {
-    if constexpr (IL) {
-      R2 v;
-      v.x = r;
-      v.y = q;
-      reinterpret_cast<R2*>(f.RU)[c + k * sk] = v;
-    } else {
-      f.RU[c + k * sk] = r;
-      f.QU[c + k * sk] = q;
-    }
+    R2 v;
+    v.x = r;
+    v.y = q;
+    reinterpret_cast<R2*>(f.RQ)[c + k * sk] = v;
   };
   auto get_rq = [&](const VdField<R>& f, int k, R& r, R& q) {
-    if constexpr (IL) {
-      const R2 v = reinterpret_cast<const R2*>(f.RU)[c + k * sk];
-      r = v.x;
-      q = v.y;
-    } else {
-      r = f.RU[c + k * sk];
-      q = f.QU[c + k * sk];
-    }
+    const R2 v = reinterpret_cast<const R2*>(f.RQ)[c + k * sk];
+    r = v.x;
+    q = v.y;
   };
   // the new value of level k from the old one and the increment: a plain FP32 sum, or the
   // compensated sum of the carried error lo (the tracer's compensated storage)

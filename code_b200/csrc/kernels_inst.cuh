@@ -290,34 +290,28 @@ int run_finalise(const Dev& d, cudaStream_t s, R dt, R* f, const R* ho, const R*
 
 template <class R>
 int run_vdiff(const Dev& d, cudaStream_t s, R dt, R cnpar, R avmol, R* S, const R* hn, const R* nuh,
-              const int32_t* az, const R* src, R* rus, R* qus, const R* Sin, R* S2, __half* lo) {
+              const int32_t* az, const R* src, R* rqs, const R* Sin, R* S2, __half* lo) {
   if (d.kmax <= 1) return 0;
   if (sizeof(R) == 8) lo = nullptr;
   const int nx = d.imax - d.imin + 1, ny = d.jmax - d.jmin + 1;
   dim3 blk(32, 4, 1);
   dim3 grd((nx + 31) / 32, (ny + 3) / 4, 1);
-  VdSet<R, 1> F{{{Sin ? Sin : S, S, src, rus, qus, S2, lo, avmol}}};
+  VdSet<R, 1> F{{{Sin ? Sin : S, S, src, rqs, S2, lo, avmol}}};
   launch_chained(k_vdiff<R, 1>, grd, blk, 0, s, d, dt, cnpar, F, hn, nuh, az, d.sk);
   return (int)cudaGetLastError();
 }
 
 template <class R>
 int run_vdiff2(const Dev& d, cudaStream_t s, R dt, R cnpar, const R* hn, const R* nuh, const int32_t* az,
-               R* Sa, R avmol_a, const R* src_a, R* rus_a, R* qus_a, __half* lo_a, R* Sb, R avmol_b, R* rus_b,
-               R* qus_b, __half* lo_b, bool hn2d) {
+               R* Sa, R avmol_a, const R* src_a, R* rqs_a, __half* lo_a, R* Sb, R avmol_b, R* rqs_b, __half* lo_b,
+               bool hn2d) {
   if (d.kmax <= 1) return 0;
   if (sizeof(R) == 8) lo_a = lo_b = nullptr;
   const int nx = d.imax - d.imin + 1, ny = d.jmax - d.jmin + 1;
   dim3 blk(32, 4, 1);
   dim3 grd((nx + 31) / 32, (ny + 3) / 4, 1);
-  VdSet<R, 2> F{{{Sa, Sa, src_a, rus_a, qus_a, nullptr, lo_a, avmol_a},
-                 {Sb, Sb, nullptr, rus_b, qus_b, nullptr, lo_b, avmol_b}}};
-  // qus_a == qus_b == nullptr: each tracer's (ru, qu) pairs interleaved in its rus array (two
-  // elements per cell): one access per level instead of two
-  if (!qus_a && !qus_b)
-    launch_chained(k_vdiff<R, 2, true>, grd, blk, 0, s, d, dt, cnpar, F, hn, nuh, az, hn2d ? 0LL : d.sk);
-  else
-    launch_chained(k_vdiff<R, 2>, grd, blk, 0, s, d, dt, cnpar, F, hn, nuh, az, hn2d ? 0LL : d.sk);
+  VdSet<R, 2> F{{{Sa, Sa, src_a, rqs_a, nullptr, lo_a, avmol_a}, {Sb, Sb, nullptr, rqs_b, nullptr, lo_b, avmol_b}}};
+  launch_chained(k_vdiff<R, 2>, grd, blk, 0, s, d, dt, cnpar, F, hn, nuh, az, hn2d ? 0LL : d.sk);
   return (int)cudaGetLastError();
 }
 
@@ -371,11 +365,11 @@ template int run_adv_pass<GB_REAL>(const Dev&, cudaStream_t, bool, int, GB_REAL,
 template int run_finalise<GB_REAL>(const Dev&, cudaStream_t, GB_REAL, GB_REAL*, const GB_REAL*, const GB_REAL*,
                                    const GB_REAL*, const uint8_t*);
 template int run_vdiff<GB_REAL>(const Dev&, cudaStream_t, GB_REAL, GB_REAL, GB_REAL, GB_REAL*, const GB_REAL*,
-                                const GB_REAL*, const int32_t*, const GB_REAL*, GB_REAL*, GB_REAL*, const GB_REAL*,
-                                GB_REAL*, __half*);
+                                const GB_REAL*, const int32_t*, const GB_REAL*, GB_REAL*, const GB_REAL*, GB_REAL*,
+                                __half*);
 template int run_vdiff2<GB_REAL>(const Dev&, cudaStream_t, GB_REAL, GB_REAL, const GB_REAL*, const GB_REAL*,
-                                 const int32_t*, GB_REAL*, GB_REAL, const GB_REAL*, GB_REAL*, GB_REAL*, __half*,
-                                 GB_REAL*, GB_REAL, GB_REAL*, GB_REAL*, __half*, bool);
+                                 const int32_t*, GB_REAL*, GB_REAL, const GB_REAL*, GB_REAL*, __half*, GB_REAL*,
+                                 GB_REAL, GB_REAL*, __half*, bool);
 template int run_tridiag<GB_REAL>(cudaStream_t, int, int, int, int, const GB_REAL*, const GB_REAL*,
                                   const GB_REAL*, const GB_REAL*, GB_REAL*);
 template int run_content<GB_REAL>(const Dev&, cudaStream_t, const GB_REAL*, const GB_REAL*, const int32_t*,

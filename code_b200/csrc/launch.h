@@ -130,24 +130,22 @@ template <class R>
 int run_finalise(const Dev& d, cudaStream_t s, R dt, R* f, const R* ho, const R* adv, const R* hi,
                  const uint8_t* mfin);
 
-// rus/qus: two scratch 3D arrays (Thomas coefficients). The old tracer is read from Sin (default:
+// rqs: scratch of 2 * sk * (kmax+1) elements (the elimination coefficients as interleaved (ru, qu)
+// pairs, one access per level). The old tracer is read from Sin (default:
 // S itself) and the new one written to S and, when given, to S2 as well; only the solved columns
 // (interior, az == 1) are written.
 template <class R>
 int run_vdiff(const Dev& d, cudaStream_t s, R dt, R cnpar, R avmol, R* S, const R* hn, const R* nuh,
-              const int32_t* az, const R* src, R* rus, R* qus, const R* Sin = nullptr, R* S2 = nullptr,
-              __half* lo = nullptr);
+              const int32_t* az, const R* src, R* rqs, const R* Sin = nullptr, R* S2 = nullptr, __half* lo = nullptr);
 
 // Two tracers (temperature a with its sources src_a, salinity b) diffused in one launch over the
-// same heights and diffusivity; each with its own molecular diffusivity, scratch pair and
+// same heights and diffusivity; each with its own molecular diffusivity, coefficient scratch and
 // compensated storage; each tracer's expressions are run_vdiff's. hn2d: hn is a 2D array of column
-// heights (every level of a column has that height). qus_a == qus_b == nullptr: each tracer's
-// elimination coefficients go to its rus array as interleaved (ru, qu) pairs (2 * sk * (kmax+1)
-// elements).
+// heights (every level of a column has that height).
 template <class R>
 int run_vdiff2(const Dev& d, cudaStream_t s, R dt, R cnpar, const R* hn, const R* nuh, const int32_t* az,
-               R* Sa, R avmol_a, const R* src_a, R* rus_a, R* qus_a, __half* lo_a, R* Sb, R avmol_b, R* rus_b,
-               R* qus_b, __half* lo_b, bool hn2d = false);
+               R* Sa, R avmol_a, const R* src_a, R* rqs_a, __half* lo_a, R* Sb, R avmol_b, R* rqs_b, __half* lo_b,
+               bool hn2d = false);
 
 template <class R>
 int run_tridiag(cudaStream_t s, int ncol, int kmax, int fi, int lt, const R* au, const R* bu, const R* cu,

@@ -125,6 +125,6 @@ extern "C" int getm_tracer_vdiff_noalloc(const getm_domain* dom, void* stream, d
   int rc = scratch_on_current_device(&scr);
   if (rc) return rc;
   const Dev d = to_dev(*dom);
-  rc = run_vdiff<double>(d, (cudaStream_t)stream, dt, cnpar, avmol, S, hn, nuh, az, src, scr, scr + kMaxCells);
+  rc = run_vdiff<double>(d, (cudaStream_t)stream, dt, cnpar, avmol, S, hn, nuh, az, src, scr);
   return rc ? GETM_ERR_CUDA : GETM_OK;
 }
