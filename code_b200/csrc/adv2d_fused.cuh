@@ -1,5 +1,5 @@
 // adv2d_fused.cuh -- the depth-averaged momentum advection of one micro step (uv_advect.F90:94-300
-// with split = HALFSPLIT) as ONE kernel per momentum component. Included by kernels_inst.cuh.
+// with split = HALFSPLIT) as ONE kernel for both momentum components. Included by kernels_inst.cuh.
 //
 // uv_advect builds the advected quantity and the face transports of the U (or V) control volumes
 // from U, V, DU, DV (uv_advect.F90:94-110 / :204-220) and runs do_advection (advection.F90:
