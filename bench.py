@@ -71,8 +71,9 @@ def stage_words(stage: str, mixed: bool, compensated: bool) -> float:
 # DRAM bytes (read + write) per interior cell per launch of the FP32 stages, averaged over the
 # stage's launches in one macro step: ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum (one
 # kernel, up to three launches) on the 1024 x 1024 x 32 case of this workload, scaled per cell
-# (w sweeps: two at 21.2 and the pair at 28.2; diffusion: one launch for T and S at 46.5).
-TRAFFIC_PER_CELL_F32 = {"adv_split_w": 23.5, "tracer_vdiff": 46.5}
+# (u/v passes: two at 20.8 and the pair at 39.6; v/u passes: two at 25.2 and the pair at 39.6; w sweeps:
+# two at 21.0 and the pair at 28.2; diffusion: one launch for T and S at 43.9).
+TRAFFIC_PER_CELL_F32 = {"adv_split_uv": 27.0, "adv_split_vu": 30.0, "adv_split_w": 23.4, "tracer_vdiff": 43.9}
 
 
 ERR_FIELDS = ("f3_T", "f3_S", "f3_uu", "f3_vv", "f2_z", "f2_U", "f2_V")
