@@ -228,7 +228,7 @@ __device__ __forceinline__ R face_cfl(bool pos, R Uf, R DUf, R dti, R cdx, R dxf
     return pos ? Uf / DUf * dti / dxf : -Uf / DUf * dti / dxf;
   } else {
     (void)dti; (void)dxf;
-    return __fdividef(fabsf(Uf) * cdx, DUf);
+    return fdiv_fast(fabsf(Uf) * cdx, DUf);
   }
 }
 
