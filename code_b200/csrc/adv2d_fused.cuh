@@ -364,10 +364,8 @@ int run_uvadv2d(const Dev& d, cudaStream_t s, T dt, int scheme, const TI* U, con
       using TL = decltype(tile);
       auto kern = k_uvadv2d_both<TL, T, S, TI>;
       const size_t smem = sizeof(Adv2dSmem<T, TL>);
-      if (smem > 48 * 1024) {  // opt-in (a host-side setting of the current device's function)
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-      }
+      if (smem > 48 * 1024)
+        if (const int e = allow_smem(kern, smem)) return e;
       const dim3 grd((d.ni() + TL::FX - 1) / TL::FX, (d.nj() + TL::FY - 1) / TL::FY, 2);
       return launch_chained(kern, grd, dim3(TL::RW, TL::FTY, 1), smem, s, d, dt, U, V, DU, DV,
                             Adv2dMasks{mu[0], mu[1], mu[2], mu[3]}, Adv2dMasks{mv[0], mv[1], mv[2], mv[3]}, UEx, VEx,

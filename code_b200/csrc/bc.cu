@@ -1103,7 +1103,7 @@ int check_state(getm_ctx* ctx, const getm_bc_state* st) {
     return fail(ctx, GETM_ERR_ARG, "ip_method must be 1..7 (internal_pressure.F90:149-168)");
   if (st->ipar[I_IP_METHOD] == 7 && ctx->dom.kmax > 64)  // the work arrays of k_svk_cols (SVK_KMAX)
     return fail(ctx, GETM_ERR_UNSUPPORTED, "ip_method 7 (STELLING_VANKESTER): at most 64 levels");
-  if ((size_t)2 * (ctx->dom.kmax + 1) * 64 * sizeof(double) > 200 * 1024)
+  if (ctx->dom.kmax > KMAX_COLUMNS)
     return fail(ctx, GETM_ERR_UNSUPPORTED, "kmax too large for the column solvers");
   return GETM_OK;
 }

@@ -876,6 +876,7 @@ __global__ void k_ip_sm(Dev d, Bc3<R3> s, const R3* zzp, const R3* Pp) {
 constexpr int UVM_SLOTS = 4;
 constexpr int UVM_IN = 9;
 constexpr int UVM_THREADS = 128;
+constexpr int UVM_SM_LEVELS = 64;  // kmax + 1 of the SM form at most
 template <class R3, int DIR, bool SM, int NT, int SL = UVM_SLOTS>
 __global__ void __launch_bounds__(NT) k_uvmom3d(Dev d, Bc3<R3> s, R3* RUs, R3* QUs) {
   chain_sync();
@@ -1716,11 +1717,10 @@ int run_bc3(int which, const Dev& d, cudaStream_t st, const Bc3<R3>& s, R3* cons
     case BC3_BF3D: launch_chained(k_bf3d<R3>, plane_grid(d, blk), blk, 0, st, d, s); break;
     case BC3_ZZ: launch_chained(k_zz<R3>, plane_grid(d, blk), blk, 0, st, d, s, scr[6]); break;
     case BC3_IP: {
-      const size_t dyn = (size_t)((d.kmax + IPG - 1) / IPG) * IPZ_H * IPZ_W * sizeof(R3);
-      if (dyn > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(k_ip<R3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-        if (e != cudaSuccess) return (int)e;
-      }
+      auto groups = [](int kmax) { return (size_t)((kmax + IPG - 1) / IPG) * IPZ_H * IPZ_W * sizeof(R3); };
+      const size_t dyn = groups(d.kmax);
+      if (dyn > 48 * 1024)
+        if (const int e = allow_smem(k_ip<R3>, groups(KMAX_COLUMNS))) return e;
       launch_chained(k_ip<R3>, plane_grid(d, blk), blk, dyn, st, d, s);
       break;
     }
@@ -1755,7 +1755,7 @@ int run_bc3(int which, const Dev& d, cudaStream_t st, const Bc3<R3>& s, R3* cons
       const int nx = d.imax - d.imin + 1, ny = d.jmax - d.jmin + 1;
       bool done = false;
       if constexpr (sizeof(R3) == 4) {
-        if (d.kmax + 1 <= 64) {
+        if (d.kmax + 1 <= UVM_SM_LEVELS) {
           constexpr int NT = 64;
           const dim3 b2(32, 2, 1);
           const dim3 g2((nx + 31) / 32, (ny + 1) / 2, 1);
@@ -1764,8 +1764,7 @@ int run_bc3(int which, const Dev& d, cudaStream_t st, const Bc3<R3>& s, R3* cons
           // in shared memory a block of 64 columns holds few warps, so each column keeps more of
           // its loads in flight; above 48 KB of shared memory per block the launch opts in
           auto kern = which == BC3_UUMOM ? k_uvmom3d<R3, 0, true, NT, 8> : k_uvmom3d<R3, 1, true, NT, 8>;
-          const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-          if (e != cudaSuccess) return (int)e;
+          if (const int e = allow_smem(kern, 2 * (size_t)UVM_SM_LEVELS * NT * sizeof(R3))) return e;
           launch_chained(kern, g2, b2, dyn, st, d, s, scr[0], scr[1]);
           done = true;
         }

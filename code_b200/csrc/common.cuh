@@ -53,6 +53,18 @@ inline int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t sm
   return (int)cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 
+// Levels that the column solvers hold in shared memory at most (getm_tridiagonal_columns, the mode-split
+// state): the limit of the entry points.
+constexpr int KMAX_COLUMNS = 199;
+
+// Before a launch of more than 48 KB of dynamic shared memory. The limit belongs to the device's function,
+// which all contexts and host threads share: `most` is the same for every launch of a kernel, since a
+// limit set to one launch's own size could be lowered by another thread before that launch.
+template <class K>
+inline int allow_smem(K* kernel, size_t most) {
+  return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+
 // Scheme ids (advection.F90:60-62)
 enum : int { NOADV = 0, UPSTREAM = 1, UPSTREAM_2DH = 2, P2 = 3, SUPERBEE = 4, MUSCL = 5, P2_PDM = 6 };
 

@@ -742,7 +742,7 @@ int getm_tridiagonal_columns(getm_ctx* ctx, int ncol, int kmax, int fi, int lt, 
   if (!ctx || ncol < 0 || kmax < 1 || fi < 0 || lt > kmax || fi >= lt || !au || !bu || !cu || !du || !value)
     return fail(ctx, GETM_ERR_ARG, "tridiagonal: bad argument");
   if (ncol == 0) return GETM_OK;
-  if ((size_t)2 * (kmax + 1) * 64 * sizeof(double) > 200 * 1024)
+  if (kmax > KMAX_COLUMNS)
     return fail(ctx, GETM_ERR_UNSUPPORTED, "tridiagonal: kmax too large");
   return cuda_fail(ctx, run_tridiag<double>(ctx->stream, ncol, kmax, fi, lt, au, bu, cu, du, value), "tridiagonal");
 }

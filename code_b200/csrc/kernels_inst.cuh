@@ -318,11 +318,9 @@ int run_vdiff2(const Dev& d, cudaStream_t s, R dt, R cnpar, const R* hn, const R
 template <class R>
 int run_tridiag(cudaStream_t s, int ncol, int kmax, int fi, int lt, const R* au, const R* bu, const R* cu,
                 const R* du, R* value) {
-  const size_t smem = 2 * (size_t)(kmax + 1) * TRN * sizeof(R);
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(k_tridiag<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-  }
+  const size_t level = 2 * TRN * sizeof(R), smem = (kmax + 1) * level;
+  if (smem > 48 * 1024)
+    if (const int e = allow_smem(k_tridiag<R>, (KMAX_COLUMNS + 1) * level)) return e;
   launch_chained(k_tridiag<R>, (ncol + TRN - 1) / TRN, TRN, smem, s, ncol, kmax, fi, lt, au, bu, cu, du, value);
   return (int)cudaGetLastError();
 }
