@@ -168,13 +168,15 @@ int do_adv3d(getm_ctx* ctx, R dt, R* f, const R* uu, const R* vv, const R* ww, c
   // diffusion 70 : 67, 317 : 275, 487 : 285; on other layouts 250x250x25 73 : 128, with diffusion 96 : 138.
   auto quads = [&](const R* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   const bool vec4 = d.sj % 4 == 0 && sk % 4 == 0 && quads(f) && quads(uu) && quads(vv) && quads(hu) && quads(hv) && quads(ho);
-  const bool worth = mom || (sizeof(R) == 8 ? n3 <= (1LL << 19) || (AH == R(0) && n3 >= (1LL << 25))
+  const bool worth = (sizeof(R) == 8 ? n3 <= (1LL << 19) || (AH == R(0) && n3 >= (1LL << 25))
                                             : !vec4 || (AH == R(0) && n3 <= (1LL << 21)));
-  const bool passes = split == GETM_HALFSPLIT && hs != NOADV && vs != NOADV && worth && two_sweeps_ok(ctx) &&
-                      apart(f, false) && apart(uu, false) && apart(vv, false) && apart(ww, false) &&
-                      apart(hu, h2d & 1u) && apart(hv, h2d & 2u) && apart(ho, h2d & 4u);
-  if (mom && (!passes || !advres || iters > 1))
+  // The momentum grids' caller has asked two_sweeps_ok before it left out the set-up pass: not asked again, as
+  // another thread may turn the switch in between.
+  if (mom && (split != GETM_HALFSPLIT || hs == NOADV || vs == NOADV || hires || !advres || iters > 1))
     return fail(ctx, GETM_ERR_STATE, "do_advection_3d: momentum advection needs the two-sweep passes");
+  const bool passes = mom || (split == GETM_HALFSPLIT && hs != NOADV && vs != NOADV && worth && two_sweeps_ok(ctx) &&
+                              apart(f, false) && apart(uu, false) && apart(vv, false) && apart(ww, false) &&
+                              apart(hu, h2d & 1u) && apart(hv, h2d & 2u) && apart(ho, h2d & 4u));
   R* H = hires && !passes ? hires : (R*)ctx->scr[1];
   const bool needs_adv = (hs != NOADV && vs != NOADV && (split == GETM_NOSPLIT || split == GETM_HVSPLIT)) ||
                          (hs != NOADV && vs == NOADV && split == GETM_NOSPLIT);
