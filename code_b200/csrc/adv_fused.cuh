@@ -12,10 +12,9 @@
 // a segment of rows of one level. In k_adv_uv the row that enters the window at j+2 is swept along i
 // first (stencil neighbours and the right face flux by warp shuffles; the outermost lanes of the warp
 // only supply them), then the four rows j-1..j+2 in registers give the flux of face j and the update
-// of row j; the row segment's first four steps only fill the window (rows = 64: 6% more row sweeps,
-// the outer lanes 6%). In k_adv_vu the v sweep of row j is followed by the u sweep of the same row. No
-// barrier and no shared-memory exchange: each thread stages the inputs of its next rows in its own
-// slots of a shared-memory ring by cp.async. Every face flux and cell update is the expression of the
+// of row j; the row segment's first four steps only fill the window (rows = 64: 6% more row sweeps). In
+// k_adv_vu the v sweep of row j is followed by the u sweep of the same row. No barrier and no shared-memory
+// exchange: each thread stages the inputs of its next rows in its own slots of a shared-memory ring by cp.async. Every face flux and cell update is the expression of the
 // one-sweep kernels (sweeps_vec.cuh), so the results equal theirs bit for bit.
 //
 // Outer lanes and rows read cells that another warp updates, so no array a launch writes may be one
@@ -30,17 +29,24 @@
 
 namespace gb {
 
-constexpr int AW = 4;  // warps per block: consecutive row segments of one strip and level
+// Warps per block: consecutive levels of one strip and row segment, which read the same masks and column
+// heights; an odd level is the only one whose block runs half empty, and those blocks come first, among
+// full ones. (Four consecutive row segments per block left three warps of four idle in domains of up to 64
+// rows: 1100x48x50 FP64 step of ten micro steps 1934 -> 1411 us. Four levels per block: the same there, but
+// up to three idle warps, 64x250x30 FP64 606 against 576 us; one level: 1024x1024x40 FP64 tracer 2711 against
+// 2671 us.)
+constexpr int AW = 2;
 
-// Blocks per SM the registers are held to: the sweeps are bound by issue and by the fixed latency of
-// dependent instructions, so warps count more than registers (2048x2048x50 mixed step, u/v passes:
-// 8.1 ms at 4 blocks, 8.8 unbounded; 1024x1024x50 FP64: 7.2 ms unbounded, 5.9 at 5 blocks, 8.0 at 6)
+// Blocks per SM the registers are held to (16 warps in FP32, 20 in FP64): the sweeps are bound by issue and by
+// the fixed latency of dependent instructions, so warps count more than registers (2048x2048x50 mixed step,
+// u/v passes: 8.1 ms at 16 warps, 8.8 unbounded; 1024x1024x50 FP64: 7.2 ms unbounded, 5.9 at 20 warps, 8.0 at 24)
 template <class R>
-constexpr int adv_blocks() { return sizeof(R) == 4 ? 4 : 5; }
+constexpr int adv_blocks() { return sizeof(R) == 4 ? 8 : 10; }
 
 // Cells a lane owns and lanes that only supply neighbours: a u sweep reads two cells to either side.
 // The second launch's v sweep must be complete on the right outer cells; with MOM = 1 each of those
-// takes the transport of the cell after it.
+// takes the transport of the cell after it. Outer lanes cost 2 of 32 with two or four cells per lane, 4 (MOM = 1
+// in the second launch: 5) with one.
 template <int N>
 struct LaneSplit {
   static constexpr int LH = N >= 2 ? 1 : 2;
@@ -303,8 +309,8 @@ struct AdvF {
   const int tid = threadIdx.y * 32 + lane;                                                       \
   const int ni = d.ni(), nj = d.nj();                                                            \
   const int c0 = (blockIdx.x * (OWN_) + lane - (LH_)) * N;                                       \
-  const int j0 = (blockIdx.y * AW + threadIdx.y) * rows;                                         \
-  if (j0 >= nj) return; /* whole warp (no barrier in these kernels) */                           \
+  const int j0 = blockIdx.y * rows, kz = nk - (int)(gridDim.z - blockIdx.z) * AW + (int)threadIdx.y; \
+  if (kz < 0) return; /* whole warp (no barrier in these kernels) */                           \
   const int j1 = min(j0 + rows, nj);                                                             \
   const bool act = c0 >= 0 && c0 < ni;                                                           \
   const int navail = act ? ni - c0 : 0;                                                          \
@@ -314,10 +320,10 @@ struct AdvF {
   const bool own = act && lane >= (LH_) && lane < (LH_) + (OWN_);                                \
   const unsigned cc = act ? c0 : 0; /* a valid column for the lanes outside the row */          \
   const unsigned sj = (unsigned)d.sj;                                                            \
-  const long long lev = (long long)blockIdx.z * d.sk;                                            \
+  const long long lev = (long long)kz * d.sk;                                                    \
   const R *const Ul = C.U + lev, *const Vl = C.V + lev;                                          \
-  const R *const DUl = C.DU + blockIdx.z * C.u.skdu, *const DVl = C.DV + blockIdx.z * C.v.skdu,  \
-          *const Dil = C.Di_src + blockIdx.z * C.u.skdi;                                         \
+  const R *const DUl = C.DU + kz * C.u.skdu, *const DVl = C.DV + kz * C.v.skdu,                  \
+          *const Dil = C.Di_src + kz * C.u.skdi;                                                 \
   auto off = [&](int j) -> unsigned { return (unsigned)min(max(j, 0), nj - 1) * sj + cc; };      \
   const bool use_AH = C.u.AH > R(0);                                                             \
   unsigned fok = 0, uok = 0; /* faces c0+m-1 and cells c0+m in the u sweep's range */           \
@@ -345,7 +351,7 @@ __device__ __forceinline__ void right_of(const R (&v)[N], R (&r)[N]) {
 }
 
 template <class R, int S, bool REC, int NF, int N, bool LO, int MOM>
-__global__ void __launch_bounds__(32 * AW, adv_blocks<R>()) k_adv_uv(Dev d, AdvC<R> C, AdvF<R, NF> F, int rows) {
+__global__ void __launch_bounds__(32 * AW, adv_blocks<R>()) k_adv_uv(Dev d, AdvC<R> C, AdvF<R, NF> F, int nk, int rows) {
   chain_sync();
   constexpr int VB = N * (int)sizeof(R);
   constexpr int LH = LaneSplit<N>::LH, OWN = 32 - LH - LaneSplit<N>::rh_uv;
@@ -547,7 +553,7 @@ __global__ void __launch_bounds__(32 * AW, adv_blocks<R>()) k_adv_uv(Dev d, AdvC
 }
 
 template <class R, int S, bool REC, int NF, int N, bool LO, int MOM>
-__global__ void __launch_bounds__(32 * AW, adv_blocks<R>()) k_adv_vu(Dev d, AdvC<R> C, AdvF<R, NF> F, int rows) {
+__global__ void __launch_bounds__(32 * AW, adv_blocks<R>()) k_adv_vu(Dev d, AdvC<R> C, AdvF<R, NF> F, int nk, int rows) {
   chain_sync();
   constexpr int VB = N * (int)sizeof(R);
   constexpr int LH = LaneSplit<N>::LH, OWN = 32 - LH - LaneSplit<N>::template rh_vu<MOM>();

@@ -1,6 +1,7 @@
 // kernels_inst.cuh -- launcher definitions; included once per precision by kernels_f64.cu and
 // kernels_f32.cu with GB_REAL defined to the arithmetic type.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <initializer_list>
 #include <type_traits>
@@ -200,9 +201,11 @@ int run_adv_pass(const Dev& d, cudaStream_t s, bool vu, int nk, R dt, int scheme
       // give fewer than 12 warps per SM
       int rows = 64;
       while (rows > 8 && strips * ((d.nj() + rows - 1) / rows) * nk < 148LL * 12) rows /= 2;
-      const dim3 blk(32, AW, 1), grd((unsigned)strips, (unsigned)((d.nj() + rows * AW - 1) / (rows * AW)), (unsigned)nk);
-      if (vu) launch_chained(k_adv_vu<R, S, REC, NF, N, LO, MOM>, grd, blk, 0, s, d, C, F, rows);
-      else launch_chained(k_adv_uv<R, S, REC, NF, N, LO, MOM>, grd, blk, 0, s, d, C, F, rows);
+      rows = std::max(rows, (d.nj() + 65534) / 65535);  // (the grid's y extent)
+      const int segs = (d.nj() + rows - 1) / rows;
+      const dim3 blk(32, AW, 1), grd((unsigned)strips, segs, (nk + AW - 1) / AW);
+      if (vu) launch_chained(k_adv_vu<R, S, REC, NF, N, LO, MOM>, grd, blk, 0, s, d, C, F, nk, rows);
+      else launch_chained(k_adv_uv<R, S, REC, NF, N, LO, MOM>, grd, blk, 0, s, d, C, F, nk, rows);
       return (int)cudaGetLastError();
     };
     using std::integral_constant;
