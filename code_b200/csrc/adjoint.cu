@@ -51,8 +51,9 @@ int ensure_adj_scratch(getm_ctx* ctx, size_t bytes) {
   return GETM_OK;
 }
 
-// Forward tracer step (HALFSPLIT, itersmax = 1) that writes the tape: the same kernels and
-// arguments as do_adv3d + vdiff_api, with branch recording switched on.
+// Forward tracer step (HALFSPLIT, itersmax = 1) that writes the tape: do_adv3d + vdiff_api with branch
+// recording switched on. Two-sweep passes or one-sweep kernels by two_sweeps_pay, whose answer may
+// differ from do_adv3d's for the same fields: both forms give the same field and branches.
 template <class R>
 int step_record(getm_ctx* ctx, R dt, R* f, const R* uu, const R* vv, const R* ww, const R* hu, const R* hv,
                 const R* ho, const R* hn, const R* nuh, int hs, int vs, R AH, R cnpar, R avmol, uint8_t* codes,
@@ -73,7 +74,7 @@ int step_record(getm_ctx* ctx, R dt, R* f, const R* uu, const R* vv, const R* ww
   const R half = R(0.5), one = R(1);
   // (level 0 of the heights is not read by the H-grid sweeps)
   const int nk = kmax;
-  if (two_sweeps_ok(ctx)) {
+  if (two_sweeps_ok(ctx) && two_sweeps_pay<R>(d, AH, false, true)) {
     TwoSweep<R> t{};
     t.flags = flags_for_tag(ctx, GETM_H_TAG);
     t.f[0] = f;

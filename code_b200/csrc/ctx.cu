@@ -159,22 +159,14 @@ int do_adv3d(getm_ctx* ctx, R dt, R* f, const R* uu, const R* vv, const R* ww, c
   auto apart = [&](const R* p, bool plane) {
     return !hires || !p || hires + n3 <= p || p + (plane ? n2d(d) : n3) <= hires;
   };
-  // A field of its own (the momentum grids' passes save their set-up pass as well): passes against
-  // one-sweep kernels, whole tracer step in us, P2_PDM. FP64: 128x128x20 70 : 91, 150x150x25 105 : 112, but
-  // 200x200x20 112 : 110, 900x120x45 566 : 459 (one-cell lanes; up to 1.45 times with diffusion, whose
-  // differences the passes form for every window row); above 2^25 elements (a field twice the L2) the halved
-  // traffic counts: 1024x1024x40 2846 : 3028, 1100x1100x50 4630 : 4536, UPSTREAM 2853 : 3144. FP32 on the vectorised one-sweep layout: 128x128x20
-  // 46 : 50, 64x446x20 54 : 65, 500x500x25 225 : 235, but 1000x800x20 535 : 521, 120x900x45 287 : 238, and with
-  // diffusion 70 : 67, 317 : 275, 487 : 285; on other layouts 250x250x25 73 : 128, with diffusion 96 : 138.
   auto quads = [&](const R* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   const bool vec4 = d.sj % 4 == 0 && sk % 4 == 0 && quads(f) && quads(uu) && quads(vv) && quads(hu) && quads(hv) && quads(ho);
-  const bool worth = (sizeof(R) == 8 ? n3 <= (1LL << 19) || (AH == R(0) && n3 >= (1LL << 25))
-                                            : !vec4 || (AH == R(0) && n3 <= (1LL << 21)));
   // The momentum grids' caller has asked two_sweeps_ok before it left out the set-up pass: not asked again, as
   // another thread may turn the switch in between.
   if (mom && (split != GETM_HALFSPLIT || hs == NOADV || vs == NOADV || hires || !advres || iters > 1))
     return fail(ctx, GETM_ERR_STATE, "do_advection_3d: momentum advection needs the two-sweep passes");
-  const bool passes = mom || (split == GETM_HALFSPLIT && hs != NOADV && vs != NOADV && worth && two_sweeps_ok(ctx) &&
+  const bool passes = mom || (split == GETM_HALFSPLIT && hs != NOADV && vs != NOADV && two_sweeps_ok(ctx) &&
+                              two_sweeps_pay<R>(d, AH, vec4, false) &&
                               apart(f, false) && apart(uu, false) && apart(vv, false) && apart(ww, false) &&
                               apart(hu, h2d & 1u) && apart(hv, h2d & 2u) && apart(ho, h2d & 4u));
   R* H = hires && !passes ? hires : (R*)ctx->scr[1];

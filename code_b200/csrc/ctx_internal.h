@@ -179,6 +179,31 @@ static inline const uint8_t* flags_for_tag(const getm_ctx* ctx, int tag) {
 static inline bool two_sweeps_ok(const getm_ctx* ctx) {
   return vector_sweeps_enabled() && ctx->dev.kmax >= 1 && ctx->dev.kmax <= 65535 && n2d(ctx->dev) < (1LL << 31);
 }
+// Whether the passes are the faster form for a single tracer (vec4: FP32 rows, levels and fields on 16-byte
+// boundaries, where the one-sweep kernels are vectorised; rec: limiter branches recorded). Small domains gain
+// from two launches fewer and from segments of 8 to 32 rows that still fill the chip once; large ones from half
+// the traffic; between 2^21 and 2^23 elements segments of 64 rows fill the chip one to two times, and the nearly
+// empty last round costs more than the passes save. Diffusion costs the passes more (its differences are
+// formed for every window row); the one-sweep kernels lose most on the layouts that their vector forms do not
+// take (FP64: odd rows). Time of the one-sweep kernels over the passes', UPSTREAM to P2_PDM [with diffusion]:
+//             tracer step                                     recorded step
+// FP64  even  <= 2^21 1.06 - 1.59 [<= 2^20 0.98 - 1.40]       0.94 - 1.53 [0.89 - 1.38]
+//             between 0.92 - 1.25 [from 2^20 0.84 - 1.10]     0.79 - 1.22 [0.73 - 1.06]
+//             >= 2^23 1.05 - 1.33 [0.96 - 1.09]               0.99 - 1.29 [0.92 - 1.08]
+//       odd   <= 2^21 1.13 - 2.04 [1.03 - 1.69]               1.08 - 1.96 [1.01 - 1.65]
+//             between 0.89 - 1.46 [0.80 - 1.24]               0.83 - 1.23 [0.77 - 1.01]
+//             >= 2^23 1.11 - 1.53 [1.01 - 1.23]               1.04 - 1.45 [0.97 - 1.24]
+// FP32  vec4  <= 2^21 1.07 - 1.35 [0.96 - 1.29]               0.98 - 1.27 [1.00 - 1.29]
+//             between 0.90 - 1.34 [0.71 - 1.21]               0.89 - 1.41 [0.89 - 1.43]
+//             >= 2^23 1.01 - 1.18 [0.83 - 1.10]               0.98 - 1.21 [0.98 - 1.21]
+//       other         1.40 - 2.50 [1.24 - 2.24]               1.39 - 2.41 [1.25 - 2.09]
+template <class R>
+static inline bool two_sweeps_pay(const gb::Dev& d, R AH, bool vec4, bool rec) {
+  const long long n3 = n3d(d);
+  const bool odd = d.sj % 2 != 0, small = n3 <= (1LL << 21), large = n3 >= (1LL << 23);
+  if (sizeof(R) == 8) return AH > R(0) && !odd ? n3 <= (1LL << 20) : small || large;
+  return rec || !vec4 || (!(AH > R(0)) && (small || large));
+}
 
 // do_advection_3d (advection_3d.F90:120-598) on device pointers; defined in ctx.cu. lo: the
 // tracer's compensated storage (FP32, FULLSPLIT / HALFSPLIT; null = none). h2d: bit 0 hu, bit 1 hv,
