@@ -51,40 +51,32 @@ __device__ __forceinline__ bool interior(const Dev& d, int i, int j) {
   return i >= d.imin && i <= d.imax && j >= d.jmin && j <= d.jmax;
 }
 
-// bottom_friction.F90:48-150: ru/rv from the depth-averaged velocities (log-law drag). Arithmetic
-// type T: FP64 in the plain step (the reference's expressions and order), FP32 in the mixed step
-// (inputs and outputs stay FP64 arrays).
-template <class T, bool MIX>
-__global__ void k_bottom_friction(Dev d, Bc2 s, Bc2W w, int runtype) {
+// bottom_friction.F90:48-150: ru/rv from the depth-averaged velocities (log-law drag), FP64: the
+// reference's expressions and order.
+static __global__ void k_bottom_friction(Dev d, Bc2 s, int runtype) {
   chain_sync();
   GB_IJ2
-  auto U = f2a<MIX, U_>(d, s, w);
-  auto V = f2a<MIX, V_>(d, s, w);
-  auto DU_ = f2a<MIX, DU>(d, s, w);
-  auto DV_ = f2a<MIX, DV>(d, s, w);
-  auto ruu = f2a<MIX, RUU>(d, s, w);
-  auto rvv = f2a<MIX, RVV>(d, s, w);
-  auto ru = f2a<MIX, RU>(d, s, w);
-  auto rv = f2a<MIX, RV>(d, s, w);
+  W2 U{d, s.f2[U_]}, V{d, s.f2[V_]}, DU_{d, s.f2[DU]}, DV_{d, s.f2[DV]}, ruu{d, s.f2[RUU]}, rvv{d, s.f2[RVV]},
+      ru{d, s.f2[RU]}, rv{d, s.f2[RV]};
   W2 zub{d, s.f2[ZUB]}, zvb{d, s.f2[ZVB]}, zub0{d, s.f2[ZUB0]}, zvb0{d, s.f2[ZVB0]};
   M2 au{d, s.au}, av{d, s.av};
-  const T kappa = T(s.par[P_KAPPA]), avmmol = T(s.par[P_AVMMOL]), min_depth = T(s.par[P_MIN_DEPTH]);
-  const T q = T(0.25), h = T(0.5);
-  auto qt = [](double a, double b) { return T(a) / T(b); };
+  const double kappa = s.par[P_KAPPA], avmmol = s.par[P_AVMMOL], min_depth = s.par[P_MIN_DEPTH];
+  const double q = 0.25, h = 0.5;
+  auto qt = [](double a, double b) { return a / b; };
   const bool in = interior(d, i, j);
   if (i <= d.imax + HALO - 1 && au(i, j) > 0) {
     // vloc: 4-point average on interior U points (0 elsewhere, as the reference's work array holds)
-    const T vloc = in ? q * (qt(V(i, j), DV_(i, j)) + qt(V(i + 1, j), DV_(i + 1, j)) + qt(V(i, j - 1), DV_(i, j - 1)) +
+    const double vloc = in ? q * (qt(V(i, j), DV_(i, j)) + qt(V(i + 1, j), DV_(i + 1, j)) + qt(V(i, j - 1), DV_(i, j - 1)) +
                              qt(V(i + 1, j - 1), DV_(i + 1, j - 1)))
-                      : T(0);
-    const T uloc = qt(U(i, j), DU_(i, j));
-    const T HHl = fmax(min_depth, T(DU_(i, j)));
-    const T zb = T(zub(i, j));
-    T x = kappa / log((zb + h * HHl) / zb);
-    T r = x * x;
+                      : 0.0;
+    const double uloc = qt(U(i, j), DU_(i, j));
+    const double HHl = fmax(min_depth, DU_(i, j));
+    const double zb = zub(i, j);
+    double x = kappa / log((zb + h * HHl) / zb);
+    double r = x * x;
     if (runtype == 1) {
-      const T fricvel = sqrt(r * (uloc * uloc + vloc * vloc));
-      const T zn = fmin(HHl, T(zub0(i, j)) + T(0.1) * avmmol / fmax(avmmol, fricvel));
+      const double fricvel = sqrt(r * (uloc * uloc + vloc * vloc));
+      const double zn = fmin(HHl, zub0(i, j) + 0.1 * avmmol / fmax(avmmol, fricvel));
       zub(i, j) = zn;
       r = (zn + h * HHl) / zn;
       x = kappa / log(r);
@@ -95,20 +87,20 @@ __global__ void k_bottom_friction(Dev d, Bc2 s, Bc2W w, int runtype) {
   }
   if (j <= d.jmax + HALO - 1 && av(i, j) > 0) {
     // uloc: 4-point average on interior V points; elsewhere the U-point quotient where au > 0
-    T uloc;
+    double uloc;
     if (in)
       uloc = q * (qt(U(i, j), DU_(i, j)) + qt(U(i - 1, j), DU_(i - 1, j)) + qt(U(i, j + 1), DU_(i, j + 1)) +
                   qt(U(i - 1, j + 1), DU_(i - 1, j + 1)));
     else
-      uloc = (i <= d.imax + HALO - 1 && au(i, j) > 0) ? qt(U(i, j), DU_(i, j)) : T(0);
-    const T vloc = qt(V(i, j), DV_(i, j));
-    const T HHl = fmax(min_depth, T(DV_(i, j)));
-    const T zb = T(zvb(i, j));
-    T x = kappa / log((zb + h * HHl) / zb);
-    T r = x * x;
+      uloc = (i <= d.imax + HALO - 1 && au(i, j) > 0) ? qt(U(i, j), DU_(i, j)) : 0.0;
+    const double vloc = qt(V(i, j), DV_(i, j));
+    const double HHl = fmax(min_depth, DV_(i, j));
+    const double zb = zvb(i, j);
+    double x = kappa / log((zb + h * HHl) / zb);
+    double r = x * x;
     if (runtype == 1) {
-      const T fricvel = sqrt(r * (uloc * uloc + vloc * vloc));
-      const T zn = fmin(HHl, T(zvb0(i, j)) + T(0.1) * avmmol / fmax(avmmol, fricvel));
+      const double fricvel = sqrt(r * (uloc * uloc + vloc * vloc));
+      const double zn = fmin(HHl, zvb0(i, j) + 0.1 * avmmol / fmax(avmmol, fricvel));
       zvb(i, j) = zn;
       r = (zn + h * HHl) / zn;
       x = kappa / log(r);
@@ -1374,8 +1366,7 @@ int bottom_friction_2d(getm_ctx* ctx, const getm_bc_state* st, int runtype, cons
   const dim3 gt((d.ni() + 31) / 32, (d.nj() + 7) / 8, 1);
   TimerScope ts(ctx, GETM_TIM_BC2D);
   if (wp) launch_chained(k_bottom_friction_f32t<true>, gt, dim3(32, 8, 1), 0, ctx->stream, d, s, w, runtype);
-  else if (st->prec3d == 8) launch_chained(k_bottom_friction<double, false>, grid2(d), kBlk2, 0, ctx->stream, d, s, w,
-                                           runtype);
+  else if (st->prec3d == 8) launch_chained(k_bottom_friction, grid2(d), kBlk2, 0, ctx->stream, d, s, runtype);
   else launch_chained(k_bottom_friction_f32t<false>, gt, dim3(32, 8, 1), 0, ctx->stream, d, s, w, runtype);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? GETM_OK : cuda_fail(ctx, (int)e, "bottom_friction");

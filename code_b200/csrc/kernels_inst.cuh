@@ -61,9 +61,10 @@ int run_sweep_h(const Dev& d, cudaStream_t s, int nk, R dt, R splitfac, int sche
     auto go = [&](auto rec, auto set) {
       constexpr bool REC = decltype(rec)::value;
       constexpr int NF = sizeof(set.t) / sizeof(set.t[0]);
-      // FP32: both directions vectorised; FP64: the v sweep (the FP64 u sweep measures faster in
-      // the tile kernel, division-bound faces)
-      const bool vec = (sizeof(R) == 4 || DIR == 1) &&
+      // FP32: both directions vectorised (a pair only with carried errors for one of the two tracers: the
+      // two-sweep passes take the others); FP64: the v sweep (the FP64 u sweep measures faster in the tile
+      // kernel, division-bound faces)
+      const bool vec = (sizeof(R) == 4 ? NF == 1 || comp : DIR == 1) &&
                        vec_layout<R>(d, nk,
                                      {set.t[0].f, set.t[0].fi_src, set.t[0].fi_dst, set.t[NF - 1].f,
                                       set.t[NF - 1].fi_src, set.t[NF - 1].fi_dst, Di_src, Di_dst, adv, U, DU},
@@ -82,10 +83,10 @@ int run_sweep_h(const Dev& d, cudaStream_t s, int nk, R dt, R splitfac, int sche
           dim3 grd((nseg + UWB - 1) / UWB, d.nj(), nz);
           SweepC<R> Cu = C;
           Cu.adv_init = adv_init && adv ? 1 : 0;
-          if (comp)
+          if (NF == 2 || comp)
             launch_chained(k_sweep_u_vec<R, S, REC, NF, true>, grd, blk, 0, s, d, Cu, nk, set, Di_src, Di_dst, adv, U,
                            DU, mflux, mupd, code);
-          else
+          else if constexpr (NF == 1)
             launch_chained(k_sweep_u_vec<R, S, REC, NF, false>, grd, blk, 0, s, d, Cu, nk, set, Di_src, Di_dst, adv,
                            U, DU, mflux, mupd, code);
           return (int)cudaGetLastError();
@@ -99,18 +100,17 @@ int run_sweep_h(const Dev& d, cudaStream_t s, int nk, R dt, R splitfac, int sche
             while (rows > 8 && nx * ((d.nj() + rows - 1) / rows) * nz * VKW < 148LL * 24) rows /= 2;
             dim3 blk(32, VKW, 1);
             dim3 grd((unsigned)nx, (d.nj() + rows - 1) / rows, (unsigned)nz);
-            if (comp)
+            if (NF == 2 || comp)
               launch_chained(k_sweep_v_vec<R, S, REC, NF, VN, true>, grd, blk, 0, s, d, C, nk, rows, set, Di_src,
                              Di_dst, adv, U, DU, mflux, mupd, code);
-            else
+            else if constexpr (NF == 1)
               launch_chained(k_sweep_v_vec<R, S, REC, NF, VN, false>, grd, blk, 0, s, d, C, nk, rows, set, Di_src,
                              Di_dst, adv, U, DU, mflux, mupd, code);
             return (int)cudaGetLastError();
           };
           // float4 lanes for one field; float2 lanes for a tracer pair (72 registers against 116:
           // measured 4% faster at 2048x2048x50 from the higher occupancy; one field measured slower)
-          if (NF == 2) return vl(std::integral_constant<int, 2>());
-          return vl(std::integral_constant<int, 4>());
+          return vl(std::integral_constant<int, NF == 2 ? 2 : 4>());
         }
       } else {
         // FP64: the j-marching v sweep on two-cell (16-byte) lanes (the 2048x2048x50 step's v

@@ -121,6 +121,25 @@ def test_macro_step_schemes(nx, scheme, dtype):
         assert np.array_equal(a[n], b[n], equal_nan=True), n
 
 
+@pytest.mark.parametrize("kept", ["Tlo", "Slo"])
+@pytest.mark.parametrize("nx", [53, 116])
+def test_pair_with_one_carried_error_array(nx, kept):
+    """The tracer pair with compensated storage of one tracer only, which keeps the one-sweep kernels."""
+    c = S.baroclinic_case(nx=nx, ny=29, kmax=6, recipe="islands", land=0.2, M=2, dt3=20.0, seed=5, dtype3=np.float32)
+    ctx, _ = make_ctx(c)
+
+    def run():
+        t = dict(BcDevice(c).t)
+        del t["f3_Slo" if kept == "Tlo" else "f3_Tlo"]
+        st = BcDevice(tensors=t, pd=dict(c.pd), pi=dict(c.pi))
+        ctx.time_loop(st, 1, 4)
+        return {n: host(a) for n, a in t.items()}
+
+    a, b = run(), _one_sweep(run)
+    for n in a:
+        assert np.array_equal(a[n], b[n], equal_nan=True), n
+
+
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
 def test_captured_steps(dtype):
     """A captured time loop and tracer step (chained launches become edges of the graph) replayed."""
