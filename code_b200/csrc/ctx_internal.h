@@ -25,7 +25,7 @@ struct getm_ctx {
   gb::Dev dev;
   cudaStream_t stream = nullptr;
   int device = 0;
-  uint8_t* planes = nullptr;   // 8 byte masks of init_advection, n2d each (see MaskPlane)
+  uint8_t* planes = nullptr;   // byte masks of init_advection, n2d each (see MaskPlane)
   int32_t* zmask = nullptr;    // copies of az, au, av (n2d each)
   bool adv_ready = false;
   void* scr[3] = {nullptr, nullptr, nullptr};  // 3D scratch: tracer ping-pong, hi, adv
@@ -131,7 +131,8 @@ static inline int cuda_fail(getm_ctx* c, int e, const char* where) {
   } while (0)
 
 // The three 3D scratch arrays, of `bytes` each (rounded up to 256) in one allocation: scr[0] and scr[1] together
-// also hold one array of twice the elements (the diffusion's coefficient pairs).
+// also hold one array of twice the elements (the diffusion's coefficient pairs). One allocation needs no more
+// room than three: the free pages it is made of need not be adjacent.
 static inline int ensure_scratch(getm_ctx* ctx, size_t bytes) {
   if (ctx->scr_bytes >= bytes) return GETM_OK;
   cudaFree(ctx->scr[0]);

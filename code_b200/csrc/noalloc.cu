@@ -1,9 +1,9 @@
 // noalloc.cu -- getm_tracer_vdiff_noalloc: the implicit vertical-diffusion solve of a tracer with
 // no context and no device allocation of any kind.
 //
-// Who needs it. getm_tracer_vdiff takes its two Thomas-coefficient scratch arrays from a context,
-// which allocates them with cudaMalloc on first use (and frees and re-allocates them when a larger
-// domain comes along). Some callers cannot accept that:
+// Who needs it. getm_tracer_vdiff takes its scratch for the Thomas coefficients from a context, which
+// allocates it with cudaMalloc on first use (and frees and re-allocates it when a larger domain comes
+// along). Some callers cannot accept that:
 //   * a host model that hands over raw device pointers and keeps no context object, e.g. a
 //     Fortran time loop that calls one C function per tracer and owns nothing else on the device;
 //   * a caller whose device memory is already committed to the model state and to other
@@ -27,8 +27,8 @@ namespace {
 
 constexpr long long kMaxCells = GETM_VDIFF_NOALLOC_MAX_CELLS;
 
-// Thomas coefficients ru (first half) and qu (second half) of every column, indexed like a 3D
-// field of the domain. Nothing here has to start at zero: in one call every thread writes the
+// Thomas coefficients of every column as (ru, qu) pairs, a pair per element of a 3D field of the
+// domain. Nothing here has to start at zero: in one call every thread writes the
 // elements of its own column before it reads them back, and reads nothing else.
 static __device__ __align__(256) double g_vdiff_scratch[2 * kMaxCells];
 

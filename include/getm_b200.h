@@ -98,8 +98,8 @@ int getm_ctx_take_warnings(getm_ctx *ctx, int64_t *n_warnings);
 #define GETM_TIM_ADV_FINALISE 3
 #define GETM_TIM_VDIFF 4
 #define GETM_TIM_COPY 5
-#define GETM_TIM_TRACER_UV 6
-#define GETM_TIM_TRACER_WVU 7
+#define GETM_TIM_TRACER_UV 6  /* two-sweep passes u/2, v/2 (momentum and tracers) */
+#define GETM_TIM_TRACER_WVU 7 /* two-sweep passes v/2, u/2 */
 #define GETM_TIM_BC2D 8  /* 2D kernels of the mode-split step */
 #define GETM_TIM_BC3D 9  /* other 3D kernels of the macro step */
 #define GETM_TIM_IP 10   /* internal pressure */
@@ -112,10 +112,11 @@ int getm_timers_reset(getm_ctx *ctx);
 int getm_timers_read(getm_ctx *ctx, int slot, double *total_ms, int64_t *launches);
 const char *getm_timer_name(int slot);
 /* Process-wide choice of the horizontal split-sweep kernels (no counterpart in the reference: a
- * tuning and testing switch). on != 0 (the default) runs the FP32 sweeps and the FP64 v sweeps in
- * the vectorised kernels wherever the rows and levels of the swept fields start on 16-byte
- * boundaries; on == 0 uses the shared-memory tile sweeps everywhere (the FP64 u sweep always
- * does). Both give identical results. Returns the previous setting. */
+ * tuning and testing switch). on != 0 (the default) runs HALFSPLIT advection as two-sweep passes
+ * where they are the faster form (momentum always), and the FP32 sweeps and the FP64 v sweeps of the
+ * rest in the vectorised kernels wherever the rows and levels of the swept fields start on 16-byte
+ * boundaries; on == 0 uses the shared-memory tile sweeps everywhere. Both give identical results; it
+ * may be turned at any time. Returns the previous setting. */
 int getm_set_vector_sweeps(int on);
 /* Process-wide choice for the mixed-precision step (no counterpart in the reference: a testing and
  * accuracy switch). on != 0 (the default) runs the barotropic micro steps of getm_time_loop on FP32
@@ -124,12 +125,12 @@ int getm_set_vector_sweeps(int on);
  * does. Returns the previous setting. */
 int getm_set_fp32_micro_steps(int on);
 /* Process-wide choice of the micro-step launches (no counterpart in the reference: a tuning and
- * testing switch). on != 0 (the default): getm_time_loop without open boundaries runs sealevel and
- * depth_update as one launch per micro step, the new elevations alternating between the z and zo
- * arrays (at the end of the call z and zo hold what the separate launches leave), forms each
- * Coriolis term inside the velocity update that reads it (the call's last term at its end), and
- * the mixed-precision micro step forms its bottom friction inside the momentum-advection kernels;
- * on == 0: the separate launches. Both give identical results. Returns the previous setting. */
+ * testing switch). on != 0 (the default): getm_time_loop runs sealevel and depth_update as one launch
+ * per micro step, the new elevations alternating between the z and zo arrays (at the end of the call
+ * z and zo hold what the separate launches leave), forms each Coriolis term inside the velocity update
+ * that reads it (the call's last term at its end), and the bottom friction inside the momentum
+ * advection's launch where that is the fused one (HALFSPLIT); on == 0: the separate launches. Both
+ * give identical results. Returns the previous setting. */
 int getm_set_fused_micro_step(int on);
 /* Human-readable text of the last error on this context (never NULL). */
 const char *getm_ctx_last_error(const getm_ctx *ctx);
