@@ -326,9 +326,10 @@ int do_adv3d_pair(getm_ctx* ctx, R dt, R* fa, R* fb, const R* uu, const R* vv, c
   const R half = R(0.5), one = R(1);
   const int nk = kmax;
   if (sizeof(R) == 8) lo_a = lo_b = nullptr;
-  // FP64: two fields' windows at 96 registers per thread lose to the one-sweep kernels where the domain
-  // fills the GPU (512x512x30: 1.02 against 0.86 ms for the four sweeps); below, four launches fewer and
-  // more warps win (step of 128x128x20: 1.43 against 1.45 ms; 200x180x25: equal)
+  // FP64: two fields' windows at 96 registers per thread (some spilled) lose to the one-sweep kernels where
+  // the domain fills the GPU; below, two launches fewer win. Step of one micro step, passes : one-sweep, us:
+  // 60x50x10 281 : 299, 128x128x20 400 : 423, 150x150x25 580 : 568, 256x256x30 1119 : 1069, 512x512x30 3605 :
+  // 3367, 120x900x45 3150 : 2695, 1024x1024x50 17061 : 16941.
   const bool small = n3d(d) <= (1LL << 19);
   if ((sizeof(R) == 4 || small) && two_sweeps_ok(ctx) && !lo_a == !lo_b && (!lo_a || lo_scr)) {
     TwoSweep<R> t{};
