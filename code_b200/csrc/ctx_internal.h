@@ -193,10 +193,10 @@ static inline bool two_sweeps_ok(const getm_ctx* ctx) {
 //             >= 2^23 1.05 - 1.33 [0.96 - 1.09]               0.99 - 1.29 [0.92 - 1.08]
 //       odd   <= 2^21 1.13 - 2.04 [1.03 - 1.69]               1.08 - 1.96 [1.01 - 1.65]
 //             between 0.89 - 1.46 [0.80 - 1.24]               0.83 - 1.23 [0.77 - 1.01]
-//             >= 2^23 1.11 - 1.53 [1.01 - 1.23]               1.04 - 1.45 [0.97 - 1.24]
+//             >= 2^23 1.11 - 1.53 [0.97 - 1.23]               1.04 - 1.45 [0.97 - 1.24]
 // FP32  vec4  <= 2^21 1.07 - 1.35 [0.96 - 1.29]               0.98 - 1.27 [1.00 - 1.29]
 //             between 0.90 - 1.34 [0.71 - 1.21]               0.89 - 1.41 [0.89 - 1.43]
-//             >= 2^23 1.01 - 1.18 [0.83 - 1.10]               0.98 - 1.21 [0.98 - 1.21]
+//             >= 2^23 0.98 - 1.18 [0.83 - 1.10]               0.98 - 1.21 [0.98 - 1.21]
 //       other         1.40 - 2.50 [1.24 - 2.24]               1.39 - 2.41 [1.25 - 2.09]
 template <class R>
 static inline bool two_sweeps_pay(const gb::Dev& d, R AH, bool vec4, bool rec) {
